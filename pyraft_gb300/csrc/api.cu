@@ -108,12 +108,11 @@ static size_t ws_total(std::initializer_list<size_t> pieces)
     return t ? Scratch::align(t) : 0;
 }
 
-// Quad scratch of the paired gathers for nz sinograms of this shape (whether
-// the geometry pairs is known only to its plan): an even view count, or (refl)
-// a backprojection's odd one.
-static size_t quads_ws(const rg_image &sino, int nz = 1, bool refl = false)
+// Quad scratch of the paired gathers for nz sinograms of this shape (an
+// even view count; whether the geometry pairs is known only to its plan).
+static size_t quads_ws(const rg_image &sino, int nz = 1)
 {
-    return refl || sino.columns % 2 == 0 ? gather_quads_bytes(sino.columns, sino.lines, nz) : 0;
+    return sino.columns % 2 == 0 ? gather_quads_bytes(sino.columns, sino.lines, nz) : 0;
 }
 
 // ----------------------------------------------------------------------------
@@ -799,17 +798,10 @@ int rg_radon_transpose_slantstack_f64(rg_image_f64 sino, rg_image_f64 image, voi
 }
 
 // ---------------------------------------------------------------- gathers
-// (A view-major sinogram of odd view count needs no workspace, as ever: its
-// backprojection stages the paired windows with loads.)
-static size_t gather_quads(const rg_image &sino, int mode)
-{
-    return quads_ws(sino, 1, mode == 0 && !is_view_major(sino));
-}
-
-static size_t gather_ws(const rg_image &sino, int mode)
+static size_t gather_ws(const rg_image &sino)
 {
     return ws_total({is_view_major(sino) ? 0 : (size_t)sino.lines * sino.columns * sizeof(float),
-                     gather_quads(sino, mode)});
+                     quads_ws(sino)});
 }
 
 static int run_gather(int mode, rg_image sino, rg_image img, void *ws, size_t wsb, void *stream)
@@ -822,14 +814,14 @@ static int run_gather(int mode, rg_image sino, rg_image img, void *ws, size_t ws
     if ((rc = get_plan(ss_geom(img, sino), 1, 0, ph))) return rc;
     const int R = sino.lines, A = sino.columns;
     Scratch s;
-    if ((rc = scratch_begin(s, ws, wsb, gather_ws(sino, mode), st))) return rc;
+    if ((rc = scratch_begin(s, ws, wsb, gather_ws(sino), st))) return rc;
     const float *s_am = sino.data;
     if (!is_view_major(sino)) {
         float *t = (float *)s.take((size_t)R * A * sizeof(float));
         rc = launch_to_am(sino.data, sino.column_stride, sino.line_stride, R, A, t, st);
         s_am = t;
     }
-    const size_t qb = gather_quads(sino, mode);
+    const size_t qb = quads_ws(sino);
     void *quads = qb ? s.take(qb) : nullptr;
     if (!rc)
         rc = autotune_gather(ph->p, mode, s_am, R, img.data, img.column_stride, img.line_stride, st,
@@ -844,7 +836,7 @@ static int run_gather(int mode, rg_image sino, rg_image img, void *ws, size_t ws
 size_t rg_backprojection_slantstack_workspace(rg_image sino, rg_image bp)
 {
     (void)bp;
-    return gather_ws(sino, 0);
+    return gather_ws(sino);
 }
 
 int rg_backprojection_slantstack(rg_image sino, rg_image bp, void *ws, size_t wsb, void *stream)
@@ -856,7 +848,7 @@ int rg_backprojection_slantstack(rg_image sino, rg_image bp, void *ws, size_t ws
 size_t rg_radon_transpose_slantstack_workspace(rg_image sino, rg_image img)
 {
     (void)img;
-    return gather_ws(sino, 1);
+    return gather_ws(sino);
 }
 
 int rg_radon_transpose_slantstack(rg_image sino, rg_image img, void *ws, size_t wsb, void *stream)
@@ -1087,7 +1079,7 @@ size_t rg_fbp_workspace(rg_image sino, rg_image image, int kind)
     (void)image;
     (void)kind;
     const size_t b = (size_t)sino.lines * sino.columns * sizeof(float);
-    return ws_total({b, b, quads_ws(sino, 1, true)});
+    return ws_total({b, b, quads_ws(sino)});
 }
 
 }  // extern "C"
@@ -1122,7 +1114,7 @@ int rg_fbp(rg_image sino, rg_image image, int kind, void *ws, size_t wsb, void *
     if ((rc = scratch_begin(s, ws, wsb, rg_fbp_workspace(sino, image, kind), st))) return rc;
     float *a = (float *)s.take((size_t)R * A * sizeof(float));
     float *b = (float *)s.take((size_t)R * A * sizeof(float));
-    const size_t qb = quads_ws(sino, 1, true);
+    const size_t qb = quads_ws(sino);
     void *quads = qb ? s.take(qb) : nullptr;
     // A small ray-major sinogram is read by the FFT filter where it lies, which
     // saves the transposing launch; its reads across the rows cost more than
@@ -1155,10 +1147,10 @@ int rg_fbp(rg_image sino, rg_image image, int kind, void *ws, size_t wsb, void *
             // gather's prepass launch is not needed
             rc = launch_filter_fft_quads(src, ivs, irs, R, A, taps->fft_p, (const float2 *)taps->p,
                                          taps->h0, taps->fft_mode,
-                                         (const View *)ph->p.d_views, (ph->p.nv + 1) / 2,
-                                         ph->p.g.A / 2, ph->p.rot_ok ? 0 : ph->p.g.A, (float4 *)quads, image.data, ph->p.g.N,
+                                         (const View *)ph->p.d_views, ph->p.nv / 2,
+                                         ph->p.g.A / 2, (float4 *)quads, image.data, ph->p.g.N,
                                          image.column_stride, image.line_stride, st,
-                                         ph->p.rot_ok && gather_quads_near(ph->p));
+                                         gather_quads_near(ph->p));
             if (!rc) {
                 QuadsPrefilled given;
                 rc = launch_gather(ph->p, 0, b, R, image.data, image.column_stride,

@@ -52,7 +52,7 @@ struct Holders {
 // Quad scratch of the paired gathers for the largest of S subsets of A views.
 static size_t em_quads_bytes(int R, int A, int S)
 {
-    return gather_quads_bytes(((A + S - 1) / S) & ~1, R, 1);   // quarter-turn pairs
+    return gather_quads_bytes((A + S - 1) / S, R, 1);
 }
 
 // Block counters of the EM update fused into the paired gathers (EmFuse).

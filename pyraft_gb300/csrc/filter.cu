@@ -425,8 +425,8 @@ __device__ __forceinline__ void fft_mid_pass(float2 *z, int p, const float2 *__r
 // against 64 bits 7.3e-6 -> 2.2e-7.
 struct FilterQuads {
     const View *views;
-    int roff, refl;        // the partner's row is view + roff, or (refl != 0) refl - view
-    int near;              // transform neighbouring rows (not with refl)
+    int roff;              // the partner's row is view + roff
+    int near;              // transform neighbouring rows
     float4 *quads;
     float *zout;
     int N;
@@ -449,11 +449,11 @@ __global__ __launch_bounds__(kFftThreads) void k_filter_fft(const float *__restr
     const bool pair = QUADS && !fq.near;             // a view and its partner
     const int a0 = pair ? fq.views[blockIdx.x].view : 2 * blockIdx.x;
     const bool circ = mode == kFilterCirc, wrap = mode == kFilterWrap;
-    const bool two = pair ? !(fq.refl && a0 == 0) : a0 + 1 < A;
+    const bool two = pair || a0 + 1 < A;
     const float *__restrict__ x = in + a0 * ivs;
     // the second row, read only when `two`
     const float *__restrict__ y =
-        in + (!pair ? a0 + 1 : fq.refl ? fq.refl - a0 : a0 + fq.roff) * ivs;
+        in + (pair ? a0 + fq.roff : a0 + 1) * ivs;
 
     // v[n] for n in [0, R), else 0
     auto v = [&](int n) {
@@ -587,23 +587,23 @@ int launch_filter_fft(const float *in, long long ivs, long long irs, float *out_
 }
 
 int launch_filter_fft_quads(const float *in, long long ivs, long long irs, int R, int A, int p, const float2 *d_tab, float g0,
-                            int mode, const View *d_views, int pairs, int roff, int refl,
+                            int mode, const View *d_views, int pairs, int roff,
                             float4 *quads, float *out, int N, long long cs, long long ls,
                             cudaStream_t st, bool near)
 {
-    if (near && (refl || 2 * roff != A || pairs != roff))
+    if (near && (2 * roff != A || pairs != roff))
         return set_error(RG_EINVAL, "filter quads: %d views do not pair by halves", A);
     if (p < 2 || p > kFilterFftMaxLog ||
         (mode == kFilterCirc ? (1 << p) != R : (1 << p) < 2 * R - 1))
         return set_error(RG_EUNSUPPORTED, "filter FFT: bad transform size 2^%d for %d rays", p, R);
-    if (pairs < 1 || (refl ? refl != A || 2 * pairs != A + 1 : roff < 1 || roff >= A))
+    if (pairs < 1 || roff < 1 || roff >= A)
         return set_error(RG_EINVAL, "filter quads: %d view pairs %d rows apart in %d views",
                          pairs, roff, A);
     const size_t smem = sizeof(float2) * (((size_t)1 << p) + ((size_t)1 << p) / 16);
     RG_CK(cudaFuncSetAttribute(k_filter_fft<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)smem));
     RG_CK(launch_pdl(k_filter_fft<true>, pairs, kFftThreads, smem, st, 1, in, ivs, irs, nullptr,
-                     R, A, p, d_tab, g0, mode, FilterQuads{d_views, roff, refl, near, quads, out, N, cs, ls}));
+                     R, A, p, d_tab, g0, mode, FilterQuads{d_views, roff, near, quads, out, N, cs, ls}));
     RG_CK_LAUNCH("k_filter_fft");
     return RG_OK;
 }

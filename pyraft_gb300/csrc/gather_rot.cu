@@ -33,18 +33,12 @@
 // both partials are added atomically: two adds onto zero give the same
 // float in either order, so the result does not depend on timing.
 //
-// Reflected views.  An odd number of views j pi / A has no quarter-turn pairs,
-// but view A - j is view j reflected: x cos(pi - theta) + y sin(pi - theta) =
-// -x cos(theta) + y sin(theta), so pixel (N-1-c, r) at view A - j meets the
-// detector where pixel (c, r) meets it at view j, at the same t and so with
-// the same validity.  The backprojection pairs those views in the same
-// kernels (refl = A): only the partner's sinogram row (A - j; view 0 has none,
-// its partner's samples are zero) and pixel differ.  These sums are kept per
-// chunk of 16 pairs and added with compensation, as in the one-view
-// gather that ran them before (without: 263 us for the first figure below and
-// four times the error).  One view / paired: 1023^2, 1155 rays x 901 views 372
-// / 298 us; 1024^2 x 721 276 / 234; 512^2 x 361 56.6 / 41.8; 256^2 x 183 18.4 /
-// 19.2, where the pairs' zeroing pass costs more than they save: from N = 384.
+// An odd number of views j pi / A has no quarter-turn pairs; its view A - j is
+// view j reflected, and pairing those (1023^2, 1155 rays x 901 views 372 -> 298
+// us) decides whether a pixel meets the detector's last sample on the rounded
+// position of another pixel: within 1e-5 of a sample of the detector's ends that
+// gains or loses whole samples against the one-view gather, 3e-3 of a Ram-Lak
+// image's rms.  So an odd count takes one view at a time.
 //
 // Staging.  When the caller supplies scratch for it, a prepass
 // (k_pair_quads) writes every quad of the plan to global memory once, [view
@@ -163,40 +157,16 @@ __device__ __forceinline__ void rot_slot(const SlotInfo &si, float P, unsigned p
     }
 }
 
-// Forms of the paired gathers (template, so that each keeps the registers it
-// has alone: with the two choices at run time the 8-row backprojection took 58
-// instead of 48, 1.785 -> 1.853 ms at 2048^2 x 1800).
-constexpr int kRot = 0;        // quarter-turn pairs
-constexpr int kRotDense = 1;   // the same on dense rays (gather_lane), backprojection
-constexpr int kRefl = 2;       // reflected pairs, backprojection, sums in chunks
-
-// kRefl: add a chunk's sums to the tile's with compensation, and clear them.
-template <int ROWS>
-__device__ __forceinline__ void rot_fold(float (&acc)[ROWS], float (&comp)[ROWS],
-                                         float (&part)[ROWS])
-{
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-        kahan_add(acc[r], comp[r], part[r]);
-        part[r] = 0.f;
-    }
-}
-
 // Add the tile's two partial sums to the output (through the cluster's
 // distributed shared memory first when the views are split over `split`
 // CTAs).  `red` is at least 2 ROWS x 256 floats of shared memory that no
 // copy writes any more; every thread of the CTA calls this.
-template <int MODE, int ROWS, int FORM>
+template <int MODE, int ROWS>
 __device__ __forceinline__ void rot_finish(const float (&accB)[ROWS], const float (&accA)[ROWS],
                                            float *red, int split, int rank, int myrow, int col,
                                            int N, float *__restrict__ out, long long cs,
                                            long long ls, float scale, bool active = true)
 {
-    // the partner's pixel: a quarter turn on, or reflected
-    auto partner = [&](int row) {
-        return FORM == kRefl ? out + (long long)row * cs + (long long)(N - 1 - col) * ls
-                             : out + (long long)col * cs + (long long)(N - 1 - row) * ls;
-    };
     if (split > 1) {
         namespace cg = cooperative_groups;
         cg::cluster_group cl = cg::this_cluster();
@@ -219,7 +189,7 @@ __device__ __forceinline__ void rot_finish(const float (&accB)[ROWS], const floa
             const bool edge = MODE != 0 && (row == 0 || col == 0 || row == N - 1 || col == N - 1);
             if (row < N && col < N && !edge) {
                 atomicAdd(out + (long long)row * cs + (long long)col * ls, sb * scale);
-                atomicAdd(partner(row), sa * scale);
+                atomicAdd(out + (long long)col * cs + (long long)(N - 1 - row) * ls, sa * scale);
             }
         }
         cl.sync();    // no CTA leaves while a peer still reads its partials
@@ -233,7 +203,7 @@ __device__ __forceinline__ void rot_finish(const float (&accB)[ROWS], const floa
         // a quarter turn maps edge pixels onto edge pixels
         if (MODE != 0 && (row == 0 || col == 0 || row == N - 1 || col == N - 1)) continue;
         atomicAdd(out + (long long)row * cs + (long long)col * ls, accB[r] * scale);
-        atomicAdd(partner(row), accA[r] * scale);
+        atomicAdd(out + (long long)col * cs + (long long)(N - 1 - row) * ls, accA[r] * scale);
     }
 }
 
@@ -351,25 +321,27 @@ __device__ __forceinline__ void rot_edges(const float *__restrict__ s_am, int s_
 
 // Warp w covers columns 8 (w & 3) .. + 8 and rows 4 ROWS (w >> 2) .. + 4
 // ROWS of the tile, 8 columns x 4 adjacent rows at a time, a lane each
-// (gather_lane, ss_tiles.cuh).
-template <int FORM> __device__ __forceinline__ int rot_lane(bool dense)
+// (gather_lane, ss_tiles.cuh).  DENSE: rays denser than pixels, a template choice
+// of the backprojection (made at run time the 8-row kernel took 58 registers
+// instead of 48, 1.785 -> 1.853 ms at 2048^2 x 1800).
+template <bool DENSE> __device__ __forceinline__ int rot_lane()
 {
-    return gather_lane(threadIdx.x & 31, FORM == kRotDense || (FORM == kRefl && dense));
+    return gather_lane(threadIdx.x & 31, DENSE);
 }
-template <int FORM> __device__ __forceinline__ int rot_cofs(bool dense)
+template <bool DENSE> __device__ __forceinline__ int rot_cofs()
 {
-    return 8 * ((threadIdx.x >> 5) & 3) + (rot_lane<FORM>(dense) & 7);
+    return 8 * ((threadIdx.x >> 5) & 3) + (rot_lane<DENSE>() & 7);
 }
-template <int FORM, int ROWS> __device__ __forceinline__ int rot_rofs(bool dense)
+template <bool DENSE, int ROWS> __device__ __forceinline__ int rot_rofs()
 {
-    return 4 * ROWS * (threadIdx.x >> 7) + (rot_lane<FORM>(dense) >> 3);
+    return 4 * ROWS * (threadIdx.x >> 7) + (rot_lane<DENSE>() >> 3);
 }
 
 // MODE 0: backprojection; MODE 1: matched adjoint (edge pixels left to the
 // edge CTAs, rot_edges, or to k_adjoint_edges, as in gather_tile with
 // edge_fixup).  Stages each chunk's
 // quads with loads from the sinogram.
-template <int MODE, int WMAX, int ROWS, bool EMF, int FORM>
+template <int MODE, int WMAX, int ROWS, bool EMF, bool DENSE>
 __device__ __forceinline__ void gather_tile_rot(const float *__restrict__ s_am, int s_ld, int R,
                                                 const View *__restrict__ views, int half,
                                                 int roff, int N, float scale,
@@ -378,8 +350,7 @@ __device__ __forceinline__ void gather_tile_rot(const float *__restrict__ s_am, 
                                                 int ty, float2 *__restrict__ pairs,
                                                 unsigned quad_bytes, int split, int rank,
                                                 float *__restrict__ em_x,
-                                                const float *__restrict__ em_inv, int *em_cnt,
-                                                int refl, bool dense)
+                                                const float *__restrict__ em_inv, int *em_cnt)
 {
     constexpr int TH = kWarps * ROWS;                     // tile height
     __shared__ SlotInfo slot[kPairSlots];
@@ -390,18 +361,13 @@ __device__ __forceinline__ void gather_tile_rot(const float *__restrict__ s_am, 
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int row0 = ty * TH, col0 = tx * kTile;
-    const int cofs = rot_cofs<FORM>(dense), rofs = rot_rofs<FORM, ROWS>(dense);
+    const int cofs = rot_cofs<DENSE>(), rofs = rot_rofs<DENSE, ROWS>();
     const int col = col0 + cofs;
     const int myrow = row0 + rofs;             // rows myrow + 4 r
 
-    constexpr bool CHUNK = FORM == kRefl;
-    float accB[ROWS], accA[ROWS], cB[CHUNK ? ROWS : 1], cA[CHUNK ? ROWS : 1];
-    float partB[CHUNK ? ROWS : 1], partA[CHUNK ? ROWS : 1];
+    float accB[ROWS], accA[ROWS];
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-        accB[r] = accA[r] = 0.f;
-        if constexpr (CHUNK) cB[r] = cA[r] = partB[r] = partA[r] = 0.f;
-    }
+    for (int r = 0; r < ROWS; ++r) { accB[r] = 0.f; accA[r] = 0.f; }
 
     const int vbeg = (int)((long long)half * rank / split);
     const int vend = (int)((long long)half * (rank + 1) / split);
@@ -425,7 +391,7 @@ __device__ __forceinline__ void gather_tile_rot(const float *__restrict__ s_am, 
                 view = v.view;
                 P = v.P;
                 d0 = v.delta;
-                if (FORM != kRefl) d1 = views[chunk + lane + half].delta;
+                d1 = views[chunk + lane + half].delta;
             }
             slot[lane] = si;
             slotW[lane] = W;
@@ -442,9 +408,7 @@ __device__ __forceinline__ void gather_tile_rot(const float *__restrict__ s_am, 
         for (int s = warp; s < nslot; s += kWarps) {
             const int nlo = slot[s].nlo, W = slotW[s];
             const float *__restrict__ rv = s_am + (size_t)slotView[s] * s_ld;
-            const int pv = FORM == kRefl ? refl - slotView[s] : slotView[s] + roff;
-            const bool alone = FORM == kRefl && slotView[s] == 0;
-            const float *__restrict__ rp = s_am + (size_t)(alone ? 0 : pv) * s_ld;
+            const float *__restrict__ rp = s_am + (size_t)(slotView[s] + roff) * s_ld;
             const float dv = slotDelta[s], dp = slotDelta[kPairSlots + s];
             for (int e = lane; e < W; e += 32) {
                 const int n = nlo + e;
@@ -452,7 +416,7 @@ __device__ __forceinline__ void gather_tile_rot(const float *__restrict__ s_am, 
                 if (MODE == 0) {
                     if (n >= 0 && n <= R - 2) {
                         const float2 a = make_pair(__ldg(rv + n), __ldg(rv + n + 1), true);
-                        const float2 b = make_pair(__ldg(rp + n), __ldg(rp + n + 1), !alone);
+                        const float2 b = make_pair(__ldg(rp + n), __ldg(rp + n + 1), true);
                         qd = make_float4(a.x, a.y, b.x, b.y);
                     }
                 } else {
@@ -470,27 +434,20 @@ __device__ __forceinline__ void gather_tile_rot(const float *__restrict__ s_am, 
             const SlotInfo si = slot[s];
             if (si.nlo == INT_MIN) continue;
             const unsigned pw = sbase + (unsigned)(s * WMAX) * quad_bytes;
-            if constexpr (CHUNK)
-                rot_slot<MODE, ROWS>(si, 0.f, pw, quad_bytes, cofs, rofs, partB, partA);
-            else
-                rot_slot<MODE, ROWS>(si, MODE == 0 ? 0.f : slotP[s], pw, quad_bytes, cofs, rofs,
-                                     accB, accA);
-        }
-        if constexpr (CHUNK) {
-            rot_fold(accB, cB, partB);
-            rot_fold(accA, cA, partA);
+            rot_slot<MODE, ROWS>(si, MODE == 0 ? 0.f : slotP[s], pw, quad_bytes, cofs, rofs,
+                                 accB, accA);
         }
         __syncthreads();
     }
     // the last chunk ended with a barrier: the staging area is free
-    rot_finish<MODE, ROWS, FORM>(accB, accA, reinterpret_cast<float *>(pairs), split, rank, myrow,
-                                 col, N, out, cs, ls, scale);
+    rot_finish<MODE, ROWS>(accB, accA, reinterpret_cast<float *>(pairs), split, rank, myrow, col,
+                           N, out, cs, ls, scale);
     if (EMF) rot_em_finish<MODE, ROWS>(row0, col0, N, out, em_x, em_inv, em_cnt, 2 * split);
 }
 
 // EMF: the EM update fused into the epilogue (EmFuse); a separate
 // instantiation, so that the plain gathers keep their registers.
-template <int MODE, int WMAX, int ROWS, bool EMF, int FORM = kRot>
+template <int MODE, int WMAX, int ROWS, bool EMF, bool DENSE = false>
 __global__ __launch_bounds__(256) void k_gather_rot(const float *__restrict__ s_am, int s_ld, int R,
                                                     const View *__restrict__ views, int half,
                                                     int roff, int N, float scale,
@@ -500,7 +457,7 @@ __global__ __launch_bounds__(256) void k_gather_rot(const float *__restrict__ s_
                                                     long long zo, unsigned quad_bytes, int split,
                                                     float *__restrict__ em_x,
                                                     const float *__restrict__ em_inv, int *em_cnt,
-                                                    int edge_rows, int refl, bool dense)
+                                                    int edge_rows)
 {
     pdl_gate();
     if (MODE == 1 && (int)blockIdx.y >= (int)gridDim.y - edge_rows) {
@@ -509,10 +466,10 @@ __global__ __launch_bounds__(256) void k_gather_rot(const float *__restrict__ s_
         return;
     }
     extern __shared__ __align__(16) float2 pairs[];  // [kPairSlots][WMAX] x {view, partner}
-    gather_tile_rot<MODE, WMAX, ROWS, EMF, FORM>(s_am + blockIdx.z * zs, s_ld, R, views, half, roff, N, scale,
+    gather_tile_rot<MODE, WMAX, ROWS, EMF, DENSE>(s_am + blockIdx.z * zs, s_ld, R, views, half, roff, N, scale,
                                 out + blockIdx.z * zo, cs, ls, err, blockIdx.x / split,
                                 blockIdx.y, pairs, quad_bytes, split, blockIdx.x % split,
-                                em_x, em_inv, em_cnt, refl, dense);
+                                em_x, em_inv, em_cnt);
 }
 
 // ---------------------------------------------------------------------------
@@ -532,7 +489,7 @@ template <int MODE>
 __global__ void k_pair_quads(const float *__restrict__ s_am, int s_ld, long long zs, int R,
                              const View *__restrict__ views, int half, int roff,
                              float4 *__restrict__ quads, float *__restrict__ zout, int N,
-                             long long cs, long long ls, long long zo, int refl)
+                             long long cs, long long ls, long long zo)
 {
     pdl_gate();
     if (zout) {
@@ -552,14 +509,11 @@ __global__ void k_pair_quads(const float *__restrict__ s_am, int s_ld, long long
     if (e >= Rq) return;
     const View &v = views[j];
     const float *__restrict__ rv = s_am + blockIdx.z * zs + (size_t)v.view * s_ld;
-    const bool alone = refl && v.view == 0;
-    const float *__restrict__ rp =
-        refl ? s_am + blockIdx.z * zs + (size_t)(alone ? 0 : refl - v.view) * s_ld
-             : rv + (size_t)roff * s_ld;
+    const float *__restrict__ rp = rv + (size_t)roff * s_ld;
     float4 qd;
     if (MODE == 0) {
         const float2 a = make_pair(__ldg(rv + e), __ldg(rv + e + 1), true);
-        const float2 b = make_pair(__ldg(rp + e), __ldg(rp + e + 1), !alone);
+        const float2 b = make_pair(__ldg(rp + e), __ldg(rp + e + 1), true);
         qd = make_float4(a.x, a.y, b.x, b.y);
     } else {
         const int n = e - 1;
@@ -586,7 +540,7 @@ __global__ void k_pair_quads(const float *__restrict__ s_am, int s_ld, long long
 // the view loop, and the CTA still takes part in its cluster's reduction.
 // expire_first (a test switch, 0 in normal use) makes the first wait give up
 // at once, so that tests can see that path run and report.
-template <int MODE, int ROWS, bool EMF, int FORM = kRot>
+template <int MODE, int ROWS, bool EMF, bool DENSE = false>
 __global__ __launch_bounds__(256) void k_gather_rot_tma(const __grid_constant__ CUtensorMap tm,
                                                         const View *__restrict__ views, int half,
                                                         int N, float scale,
@@ -600,7 +554,7 @@ __global__ __launch_bounds__(256) void k_gather_rot_tma(const __grid_constant__ 
                                                         int *em_cnt,
                                                         const float *__restrict__ s_am, int s_ld,
                                                         int R, long long zs, int edge_rows,
-                                                        int nfull, int nhalf, bool dense)
+                                                        int nfull, int nhalf)
 {
     pdl_gate();
     if (MODE == 1 && (int)blockIdx.y >= (int)gridDim.y - edge_rows) {
@@ -639,18 +593,13 @@ __global__ __launch_bounds__(256) void k_gather_rot_tma(const __grid_constant__ 
     const int z = blockIdx.z;
     out += (long long)z * zo;
     const int row0 = ty * TH, col0 = tx * kTile;
-    const int cofs = rot_cofs<FORM>(dense), rofs = rot_rofs<FORM, ROWS>(dense);
+    const int cofs = rot_cofs<DENSE>(), rofs = rot_rofs<DENSE, ROWS>();
     const int col = col0 + cofs;
     const int myrow = row0 + rofs;
 
-    constexpr bool CHUNK = FORM == kRefl;
-    float accB[ROWS], accA[ROWS], cB[CHUNK ? ROWS : 1], cA[CHUNK ? ROWS : 1];
-    float partB[CHUNK ? ROWS : 1], partA[CHUNK ? ROWS : 1];
+    float accB[ROWS], accA[ROWS];
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-        accB[r] = accA[r] = 0.f;
-        if constexpr (CHUNK) cB[r] = cA[r] = partB[r] = partA[r] = 0.f;
-    }
+    for (int r = 0; r < ROWS; ++r) { accB[r] = 0.f; accA[r] = 0.f; }
 
     const int vbeg = (int)((long long)half * rank / split);
     const int vend = (int)((long long)half * (rank + 1) / split);
@@ -714,15 +663,8 @@ __global__ __launch_bounds__(256) void k_gather_rot_tma(const __grid_constant__ 
             const SlotInfo si = slot[b][s];
             if (si.nlo == INT_MIN) continue;
             const unsigned pw = qbase + (unsigned)(b * kPairSlots + s) * slot_bytes;
-            if constexpr (CHUNK)
-                rot_slot<MODE, ROWS>(si, 0.f, pw, quad_bytes, cofs, rofs, partB, partA);
-            else
-                rot_slot<MODE, ROWS>(si, MODE == 0 ? 0.f : slotP[b][s], pw, quad_bytes, cofs,
-                                     rofs, accB, accA);
-        }
-        if constexpr (CHUNK) {
-            rot_fold(accB, cB, partB);
-            rot_fold(accA, cA, partA);
+            rot_slot<MODE, ROWS>(si, MODE == 0 ? 0.f : slotP[b][s], pw, quad_bytes, cofs, rofs,
+                                 accB, accA);
         }
         // closes chunk c: every thread is done with its buffer and slots
         if (__syncthreads_or(!ok)) {
@@ -739,8 +681,8 @@ __global__ __launch_bounds__(256) void k_gather_rot_tma(const __grid_constant__ 
         }
         __syncthreads();
     }
-    rot_finish<MODE, ROWS, FORM>(accB, accA, reinterpret_cast<float *>(qbuf), split, rank, myrow,
-                                 col, N, out, cs, ls, scale, active);
+    rot_finish<MODE, ROWS>(accB, accA, reinterpret_cast<float *>(qbuf), split, rank, myrow, col,
+                           N, out, cs, ls, scale, active);
     if (EMF) rot_em_finish<MODE, ROWS>(row0, col0, N, out, em_x, em_inv, em_cnt, 2 * split);
 }
 
@@ -762,16 +704,14 @@ int gather_rot_w(const SSPlan &p, const float *s_am, int s_ld, float *out, long 
     const float *ei = em ? em->inv : nullptr;
     int *ec = em ? em->cnt : nullptr;
     // half: view pairs; roff: sinogram rows between a view and its partner
-    const int N = p.g.N, half = (p.nv + 1) / 2, roff = p.g.A / 2, refl = p.rot_ok ? 0 : p.g.A;
+    const int N = p.g.N, half = p.nv / 2, roff = p.g.A / 2;
     // the staging area, which also holds the cluster reduction's partials
     const size_t smem = std::max((size_t)kPairSlots * WMAX * sizeof(float4),
                                  (size_t)2 * ROWS * 256 * sizeof(float));
     dim3 grid((N + kTile - 1) / kTile, (N + kWarps * ROWS - 1) / (kWarps * ROWS), z.n);
     auto k = em ? k_gather_rot<MODE, WMAX, ROWS, true> : k_gather_rot<MODE, WMAX, ROWS, false>;
     if constexpr (MODE == 0)
-        if (!em && (refl || p.dense))
-            k = refl ? k_gather_rot<0, WMAX, ROWS, false, kRefl>
-                     : k_gather_rot<0, WMAX, ROWS, false, kRotDense>;
+        if (!em && p.dense) k = k_gather_rot<0, WMAX, ROWS, false, true>;
     RG_CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int split = gather_pick_split((const void *)k, smem, ROWS, half, grid, st);
     const unsigned pb = (unsigned)sizeof(float4);
@@ -779,8 +719,7 @@ int gather_rot_w(const SSPlan &p, const float *s_am, int s_ld, float *out, long 
     const int er = edge_rows_for(N, (int)grid.x * split, MODE == 1 && edges);
     RG_CK(launch_pdl(k, dim3(grid.x * split, grid.y + er, grid.z), 256, smem, st, split,
                      s_am, s_ld, p.g.R, (const View *)p.d_views, half, roff, N,
-                     scale, out, cs, ls, d_err, z.in, z.out, pb, split, ex, ei, ec, er, refl,
-                     p.dense));
+                     scale, out, cs, ls, d_err, z.in, z.out, pb, split, ex, ei, ec, er));
     RG_CK_LAUNCH("k_gather_rot");
     return RG_OK;
 }
@@ -818,13 +757,12 @@ int gather_rot_tma(const SSPlan &p, const float *s_am, int s_ld, float *out, lon
     float *ex = em ? em->x : nullptr;
     const float *ei = em ? em->inv : nullptr;
     int *ec = em ? em->cnt : nullptr;
-    const int N = p.g.N, R = p.g.R, half = (p.nv + 1) / 2, roff = p.g.A / 2;
-    const int refl = p.rot_ok ? 0 : p.g.A;
+    const int N = p.g.N, R = p.g.R, half = p.nv / 2, roff = p.g.A / 2;
     const int Rq = quad_entries(MODE, R);
     if (!(MODE == 0 && t_quads_prefilled)) {
         dim3 g((Rq + 255) / 256, half, z.n);
         RG_CK(launch_pdl(k_pair_quads<MODE>, g, 256, 0, st, 1, s_am, s_ld, z.in, R, p.d_views,
-                         half, roff, quads, zero_out ? out : nullptr, N, cs, ls, z.out, refl));
+                         half, roff, quads, zero_out ? out : nullptr, N, cs, ls, z.out));
         RG_CK_LAUNCH("k_pair_quads");
     }
     // RG_TEST_WINDOW_CUT=1 (a test switch) under-reports the window bound by
@@ -848,9 +786,7 @@ int gather_rot_tma(const SSPlan &p, const float *s_am, int s_ld, float *out, lon
     }
     auto k = em ? k_gather_rot_tma<MODE, ROWS, true> : k_gather_rot_tma<MODE, ROWS, false>;
     if constexpr (MODE == 0)
-        if (!em && (refl || p.dense))
-            k = refl ? k_gather_rot_tma<0, ROWS, false, kRefl>
-                     : k_gather_rot_tma<0, ROWS, false, kRotDense>;
+        if (!em && p.dense) k = k_gather_rot_tma<0, ROWS, false, true>;
     // two buffers of 16 windows, which also hold the cluster reduction's partials
     const size_t smem = std::max((size_t)kStages * kPairSlots * wb * sizeof(float4),
                                  (size_t)2 * ROWS * 256 * sizeof(float));
@@ -878,15 +814,15 @@ int gather_rot_tma(const SSPlan &p, const float *s_am, int s_ld, float *out, lon
     RG_CK(launch_pdl(k, dim3(g.x * split, g.y + er, g.z), 256, smem, st, split,
                      tm, (const View *)p.d_views, half, N, scale, out, cs, ls,
                      d_err, z.out, wb, qb, split, expire, ex, ei, ec, s_am, s_ld, R, z.in, er,
-                     nfull, nhalf, p.dense));
+                     nfull, nhalf));
     RG_CK_LAUNCH("k_gather_rot_tma");
     return RG_OK;
 }
 
 // Whether the paired gathers of nz slices stage by TMA where the call brings the
 // quad scratch (RG_GATHER_ROT_TMA: 0 never, 1 always).  From 256 view pairs
-// always.  Below, quarter-turn pairs only, by the work (pixels x pairs), loads
-// / TMA in us: the prepass must be made up for.  Adjoint 512^2 x 180 pairs 48.1
+// always.  Below, by the work (pixels x pairs), loads / TMA in us: the prepass
+// must be made up for.  Adjoint 512^2 x 180 pairs 48.1
 // / 49.0, x 250 61.3 / 59.5, 1024^2 x 90 78.8 / 76.0, x 180 137 / 126, 2048^2 x
 // 180 463 / 416, a stack of 8 512^2 x 180 294 / 273 (x 90 168 / 171).
 // Backprojection 512^2 x 180 48 / 46, 1024^2 x 180 121 / 126, x 250 159 / 161,
@@ -899,9 +835,8 @@ bool gather_rot_use_tma(const SSPlan &p, int mode, int nz, bool prefilled)
     const char *e = getenv("RG_GATHER_ROT_TMA");
     if (e && !strcmp(e, "0")) return false;
     if (e && !strcmp(e, "1")) return true;
-    const int pairs = (p.nv + 1) / 2;
+    const int pairs = p.nv / 2;
     if (pairs >= kTmaMinPairs) return true;
-    if (!p.rot_ok) return false;
     const double work = (double)nz * p.g.N * p.g.N * pairs;
     if (mode == 1) return pairs >= 128 ? work >= 64e6 : pairs >= 90 && nz == 1 && work >= 90e6;
     return (prefilled && work <= 11e6) || (pairs >= 128 && work >= 700e6);
@@ -912,7 +847,7 @@ bool tma_form(const SSPlan &p, int mode, int rows, bool quads, int nz, bool pref
 {
     const int t = rows == 16 ? 2 : rows == 8 ? 1 : 0;
     const int w = mode == 0 ? p.wmax_bp[t] : p.wmax_adj[t];
-    const int pairs = (p.nv + 1) / 2;
+    const int pairs = p.nv / 2;
     return quads && quad_box(w) <= kQuadBox && pairs <= 65535 &&
            gather_rot_use_tma(p, mode, nz, prefilled);
 }
@@ -951,11 +886,11 @@ QuadsPrefilled::~QuadsPrefilled() { t_quads_prefilled = false; }
 
 bool gather_quads_form(const SSPlan &p, void *quads)
 {
-    return quads && (p.rot_ok || p.refl_ok) && gather_rot_enabled() && 
+    return quads && p.rot_ok && gather_rot_enabled() &&
            tma_form(p, 0, tuned_rows(p, 0), true, 1, true);
 }
 
-bool gather_quads_near(const SSPlan &p) { return (p.nv + 1) / 2 < kTmaMinPairs; }
+bool gather_quads_near(const SSPlan &p) { return p.nv / 2 < kTmaMinPairs; }
 
 int launch_zero_image(float *out, int N, long long cs, long long ls, cudaStream_t st,
                       const Stack &z)
@@ -970,7 +905,7 @@ int launch_zero_image(float *out, int N, long long cs, long long ls, cudaStream_
 size_t gather_quads_bytes(int nv, int R, int nz)
 {
     if (nv < 2 || R < 2 || nz < 1) return 0;
-    return (size_t)nz * (size_t)((nv + 1) / 2) * (size_t)quad_entries(1, R) * sizeof(float4);
+    return (size_t)nz * (size_t)(nv / 2) * (size_t)quad_entries(1, R) * sizeof(float4);
 }
 
 int launch_gather_rot(const SSPlan &p, int mode, const float *s_am, int s_ld, float *out,

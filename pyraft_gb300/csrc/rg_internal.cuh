@@ -198,8 +198,6 @@ struct SSPlan {
     bool contiguous = true;        // views are consecutive (not an OSEM subset)
     bool rot_ok = false;           // second half of the views = first half + pi/2, on a grid
                                    // symmetric under a quarter turn (gather_rot.cu)
-    bool refl_ok = false;          // view A - j is view j reflected (theta = j pi / A, A odd), on a
-                                   // grid symmetric in x (gather_rot.cu)
     bool mirror_ok = false;        // image and detector centred on 0: pixel (r, c) and
                                    // (N-1-r, N-1-c) meet a view at mirrored ray positions
                                    // (gather_tile_mirror)
@@ -342,8 +340,7 @@ int launch_gather(const SSPlan &p, int mode, const float *s_am, int s_ld,
 int launch_sens(const SSPlan &p, const float *ones_am, int s_ld, float *inv, float *scratch,
                 cudaStream_t st);
 // Bytes of the paired gathers' quad scratch for nz problems of nv views over
-// R rays: a 16-byte quad per (view pair, sample entry), R + 1 entries (an odd
-// view out pairs with nothing).
+// R rays: a 16-byte quad per (view pair, sample entry), R + 1 entries.
 size_t gather_quads_bytes(int nv, int R, int nz);
 // The gather launch shape picked for (geometry, mode) by the autotuner
 // (api.cu): rows per thread and the cluster view split (0: the occupancy
@@ -378,8 +375,7 @@ struct SplitPref {
     int saved;
 };
 // Backprojection (mode 0) or matched adjoint (mode 1) with views paired a
-// quarter turn apart (p.rot_ok), or the backprojection with reflected views
-// paired (p.refl_ok).  Two partial sums are added to each
+// quarter turn apart (p.rot_ok).  Two partial sums are added to each
 // interior pixel of an output that is zeroed first: by this call when
 // zero_out (in the quad prepass where it runs), else by the caller.  The
 // adjoint's edge pixels are computed by extra CTAs of the same launch when
@@ -460,11 +456,11 @@ enum { kFilterLinear = 0, kFilterCirc = 1, kFilterWrap = 2 };
 int launch_filter_fft(const float *in, long long ivs, long long irs, float *out_am, int R, int A, int p, const float2 *d_tab,
                       float g0, int mode, cudaStream_t st);
 // The same filter for the FBP: CTA j filters rows v = d_views[j].view and v +
-// roff (refl: A - v, and row 0 alone) of in_am (j < pairs) and writes the paired
+// roff of in (j < pairs; near: rows 2j and 2j + 1) and writes the paired
 // backprojection's quads[j][e] (e < R - 1) instead of the rows, and the CTAs
 // zero the N x N output (strides cs, ls).
 int launch_filter_fft_quads(const float *in, long long ivs, long long irs, int R, int A, int p, const float2 *d_tab, float g0,
-                            int mode, const View *d_views, int pairs, int roff, int refl,
+                            int mode, const View *d_views, int pairs, int roff,
                             float4 *quads, float *out, int N, long long cs, long long ls,
                             cudaStream_t st, bool near);
 

@@ -145,12 +145,6 @@ int ss_views_compute(SSPlan &p, const SSGeom &g, const int *views, int nv, View 
     const double pi = 3.14159265358979323846;
     p.rot_ok = nv >= 2 && nv % 2 == 0 && g.A % 2 == 0 && fabs((thf - th0) - pi) <= 1e-12 * pi &&
                g.itl_x == g.ibr_y && g.ibr_x == g.itl_y && g.itl_x == -g.ibr_x;
-    // Views theta = j pi / A, all of them, in an odd count (an even one pairs a
-    // quarter turn apart): view A - j at -x is view j at x.
-    // (N: where the pairs are the faster form, gather_rot.cu)
-    p.refl_ok = g.N >= 384 && g.A % 2 == 1 && nv == g.A && nv >= 3 && th0 == 0.0 &&
-                fabs(thf - pi) <= 1e-12 * pi && g.itl_x == -g.ibr_x;
-    for (int e = 0; e < nv && p.refl_ok; ++e) p.refl_ok = (views ? views[e] : e) == e;
     // A half turn maps the grid onto itself and t onto -t: x and y each
     // centred on 0, and the detector's t range centred on 0.
     p.mirror_ok = g.itl_x == -g.ibr_x && g.itl_y == -g.ibr_y && g.stl_y == -g.sbr_y;
@@ -770,7 +764,7 @@ int launch_gather(const SSPlan &p, int mode, const float *s_am, int s_ld, float 
         ef.inv = inv_sens;
     }
     if (mode == 0) {
-        if (!em_x && (p.rot_ok || p.refl_ok) && gather_rot_enabled())
+        if (!em_x && p.rot_ok && gather_rot_enabled())
             return launch_gather_rot(p, 0, s_am, s_ld, out, cs, ls, d_err, st, rows, z, quads,
                                      true);
         if (fused)
