@@ -27,15 +27,17 @@
 // a strip that would not fit is skipped with an error flag, never read out
 // of bounds.  The window holds the positions of all the CTA's rays on all 16
 // lines, on the image or off it, and holds zeros off it: so a warp walks a
-// strip whole or not at all, and no ray's first and last line are computed
-// (lanes that start or end inside a strip each took a loop of their own: 512^2
-// x 360 53 -> 47.6 us, DDA 61 -> 54 us, 2048^2 x 1800 unchanged).  The plan also fixes the order in which the (ray tile, view
-// block) CTAs are dispatched, most strips first (st_cta_order), so that the
-// launch's last wave holds its lightest CTAs, and each CTA's range of strips,
-// so that the first load starts before anything else.  One barrier closes a
-// strip.  Every mbarrier wait is
-// bounded; a CTA whose wait runs out sets
-// the error flag, waits (bounded) for its own copies and leaves.
+// strip whole or not at all (lanes that start or end inside a strip each took a
+// loop of their own: 512^2 x 360 53 -> 47.6 us, DDA 61 -> 54 us).  A slant-stack
+// ray's run of strips is known from the start (ray_strips): the vote on a strip
+// is two comparisons, where those of its two end positions took a twelfth of
+// the kernel (2048^2 x 1800 2.05 -> 1.90 ms).  The plan also fixes the order in
+// which the (ray tile, view block) CTAs are dispatched, most strips first
+// (st_cta_order), so that the launch's last wave holds its lightest CTAs, and
+// each CTA's range of strips, so that the first load starts before anything
+// else.  One barrier closes a strip.  Every mbarrier wait is bounded; a CTA
+// whose wait runs out sets the error flag, waits (bounded) for its own copies
+// and leaves.
 // expire_first (a test switch, 0 in normal use) makes each CTA's first strip
 // wait give up at once, so that tests can see that path run and report.
 #include <cuda.h>
@@ -89,6 +91,41 @@ __device__ __forceinline__ void strip16(unsigned sb, unsigned &L, unsigned dq, u
         L += dq;
         strip16<BW, R0 + 1, DDA>(sb, L, dq, pb, wa, wc, part, odd);
     }
+}
+
+// Slant stack: the run of strips that a ray walks, from that of its first line on
+// the image (bits 8 and up of `first`) to that of its last, by radon_line_range
+// (whose check of the ends cannot fail here, where a strip's positions fit a
+// window).
+//
+// A sample counts while its floor index is in [0, N - 2], and its value does not
+// vanish at the ends, so it is one position that decides, to the last bit: on
+// every strip the Q9.23 one that starts truncated at the ray's first line there
+// and steps on.  That is the strip's first line but on the strip where the ray
+// comes in; the low byte of `first` is the difference there, plus 128, between
+// the position that starts at the ray's first line, brought back to the
+// strip's, and the one that starts at the strip's (lines before the ray's first
+// read zeros).  Positions centred on a strip give and take single samples.
+__device__ __forceinline__ void ray_strips(long long u0, long long q, int N, unsigned &first,
+                                           unsigned &last)
+{
+    const float uf = (float)u0 * 2.3283064365386963e-10f, qf = (float)q * 2.3283064365386963e-10f;
+    int lo = 0, hi = N - 1;
+    if (fabsf(qf) < 1e-20f) {
+        if (!(uf >= -0.5f && uf <= (float)N - 0.5f)) hi = -1;
+    } else {
+        const float t1 = (-0.5f - uf) / qf, t2 = ((float)N - 0.5f - uf) / qf;
+        lo = (int)ceilf(fmaxf(fminf(t1, t2), 0.f));
+        hi = (int)floorf(fminf(fmaxf(t1, t2), (float)(N - 1)));
+    }
+    first = 0x7FFFFF00u;                              // no strip
+    last = 0;
+    if (lo > hi) return;
+    const int m = lo & (kTmLines - 1);
+    const long long ua = u0 + (long long)(lo - m) * q;
+    const int c = (int)((ua + m * q) >> 9) - (int)(ua >> 9) - m * (int)((q + 256) >> 9);
+    first = ((unsigned)lo / kTmLines << 8) | (unsigned)(c + 128);
+    last = (unsigned)hi / kTmLines;
 }
 
 // Lane layout: each shared load of a warp covers RPL consecutive rays of
@@ -221,6 +258,7 @@ __global__ __launch_bounds__(256, 3) void k_radon_tma(const __grid_constant__ CU
     // Threads past the block's views or the last ray walk the last ones again
     // (their windows hold no others) and store nothing.
     long long u0[kTmVpt], q[kTmVpt];
+    unsigned first[kTmVpt], last[kTmVpt];             // slant stack: ray_strips
     // all four pairs of a thread are of one view at 8 rays per load
     static_assert(!DDA || RPL == 8, "the DDA form keeps one trapezoid per thread");
     float wa = 0.f, wc = 0.f;
@@ -232,6 +270,8 @@ __global__ __launch_bounds__(256, 3) void k_radon_tma(const __grid_constant__ CU
         if constexpr (DDA) {
             wa = V.wa;
             wc = fmaf(-2.f, wa, 1.f);                 // exact
+        } else {
+            ray_strips(u0[v], q[v], N, first[v], last[v]);
         }
     }
     float acc[kTmVpt], comp[kTmVpt];
@@ -259,23 +299,31 @@ __global__ __launch_bounds__(256, 3) void k_radon_tma(const __grid_constant__ CU
             for (int v = 0; v < kTmVpt; ++v) {
                 // All 16 lines, for the whole warp, where any of its rays meets the
                 // strip: samples off the line or past the last line read zeros
-                // (the window covers every position of the CTA's rays), so no
-                // ray's first and last line are needed.
+                // (the window covers every position of the CTA's rays).
                 const long long ua = u0[v] + (long long)i0 * q[v];
-                const long long ub = ua + (kTmLines - 1) * q[v];
-                if (!__any_sync(0xffffffffu, max(ua, ub) >= -(1LL << Q) &&
-                                                 min(ua, ub) < (long long)ne << Q))
-                    continue;
-                // The rounding of the Q9.23 step is spread evenly about the strip's
-                // middle line instead of growing along it.  (The slant stack's
-                // origin is truncated: a sample just inside its line's end must
-                // not round onto it, where it would not count.)
+                unsigned shift = 0;                   // under 256: the ray comes in here
+                bool meets;
+                if constexpr (DDA) {
+                    const long long ub = ua + (kTmLines - 1) * q[v];
+                    meets = max(ua, ub) >= -(1LL << Q) && min(ua, ub) < (long long)ne << Q;
+                } else {
+                    shift = first[v] - ((unsigned)i0 / kTmLines << 8);
+                    meets = (int)shift < 256 && (unsigned)i0 / kTmLines <= last[v];
+                }
+                if (!__any_sync(0xffffffffu, meets)) continue;
                 const long long dq64 = (q[v] + (1LL << (Q - 24))) >> (Q - 23);
                 const unsigned dq = (unsigned)dq64;
-                unsigned L = (unsigned)((ua - ((long long)(x0 - 1) << Q) +
-                                         (DDA ? 1LL << (Q - 24) : 0LL) +
-                                         ((q[v] - (dq64 << (Q - 23))) * (kTmLines - 1) >> 1)) >>
-                                        (Q - 23));
+                unsigned L;
+                if constexpr (DDA) {
+                    // The rounding of the Q9.23 step is spread evenly about the
+                    // strip's middle line instead of growing along it.
+                    L = (unsigned)((ua - ((long long)(x0 - 1) << Q) + (1LL << (Q - 24)) +
+                                    ((q[v] - (dq64 << (Q - 23))) * (kTmLines - 1) >> 1)) >>
+                                   (Q - 23));
+                } else {
+                    L = (unsigned)((ua - ((long long)(x0 - 1) << Q)) >> (Q - 23));
+                    if (shift < 256u) L += shift - 128u;
+                }
                 float part = 0.f, odd = 0.f;
                 strip16<BW, 0, DDA>(sb, L, dq, pb, wa, wc, part, odd);
                 kahan_add(acc[v], comp[v], part);

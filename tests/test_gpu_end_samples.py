@@ -66,3 +66,43 @@ def test_backprojection_element_by_element(orc, monkeypatch, n, r, a, rows):
     if a % 2:
         monkeypatch.setenv("RG_GATHER_ROT", "0")
         assert np.array_equal(got, run())
+
+
+def _line_counts(n, r, a, e, j):
+    """Samples of view j's rays that the Radon counts: on each strip of 16 lines
+    positions start from the truncated Q32.32 one of the ray's first line in the
+    strip and step in units of 2^-23."""
+    d, dt = 2.0 * e / (n - 1), 2.0 / (r - 1)
+    th = j * (math.pi / a)
+    c, s, tn = math.cos(th), math.sin(th), math.tan(th)
+    if abs(c) < 1.0 / math.sqrt(2.0):
+        rk, ri, r0 = dt / (s * d), -d / (tn * d), (-1.0 / s + e / tn + e) / d
+    else:
+        rk, ri, r0 = dt / (c * d), -d * tn / d, (-1.0 / c + e * tn + e) / d
+    rk, ri, r0 = (int(round(v * 4294967296.0)) for v in (rk, ri, r0))
+    u0 = r0 + np.arange(r, dtype=np.int64)[:, None] * rk
+    i = np.arange(n, dtype=np.int64)[None, :]
+    # lines within [-0.5, n - 0.5], as estimated in FP32
+    f = np.float32
+    uf, qf = u0.astype(f) * f(2.0 ** -32), f(f(ri) * f(2.0 ** -32))
+    t1, t2 = (f(-0.5) - uf) / qf, (f(n) - f(0.5) - uf) / qf
+    lo = np.ceil(np.maximum(np.minimum(t1, t2), f(0))).astype(np.int64)
+    hi = np.floor(np.minimum(np.maximum(t1, t2), f(n - 1))).astype(np.int64)
+    first = np.maximum(lo, i & ~15)
+    k = (((u0 + first * ri) >> 9) + (i - first) * ((ri + 256) >> 9)) >> 23
+    return ((i >= lo) & (i <= hi) & (k >= 0) & (k <= n - 2)).sum(1), d / max(abs(c), abs(s))
+
+
+@pytest.mark.parametrize("n,r,a,e,views", [
+    (1205, 1450, 851, 1.0, [305, 40, 422, 700]), (1205, 1450, 851, 0.6, [29, 822, 60, 500]),
+    (333, 401, 97, 0.75, range(1, 97, 5))])
+def test_radon_counts_the_samples_of_truncated_positions(n, r, a, e, views):
+    """Of an image of ones a ray's sum is its step times the samples it counts.
+    Views 305 (ray 1205) and 29 and 822 (ray 248) meet a line's end so closely
+    that positions rounded about the strip's middle count another number."""
+    g = rg.gpu_image(torch.ones((n, n), device="cuda"), (-e, e), (e, -e))
+    got = rg.radon(g, (r, a), SLANT).data.cpu().numpy().astype(np.float64)
+    for j in views:
+        want, step = _line_counts(n, r, a, e, j)
+        assert np.array_equal(np.rint(got[:, j] / step), want)
+        assert np.max(np.abs(got[:, j] / step - want)) < 0.01
