@@ -176,10 +176,12 @@ static int em_ss_core(const SSGeom &g, long long first, long long count, int S,
     for (int k = 0; k < S; ++k) any_rot = any_rot || plans[k]->rot_ok;
     const bool fused = any_rot && gather_rot_enabled() && em_fusable(N) && !em_unfused();
     // launch shape of each plan's gathers: timed on the first run of a
-    // geometry outside a stream capture, on gsum (zeroed below)
+    // geometry outside a stream capture, on gsum (zeroed below).  The quad
+    // scratch holds quarter-turn pairs: no other form may stage in it.
     int rc = RG_OK;
     for (int k = 0; k < S && !rc; ++k)
-        rc = autotune_gather(*plans[k], bp ? 0 : 1, y_am, R, gsum, N, 1, st, quads);
+        rc = autotune_gather(*plans[k], bp ? 0 : 1, y_am, R, gsum, N, 1, st,
+                             plans[k]->rot_ok ? quads : nullptr);
     if (!rc) rc = launch_fill(ratio, (size_t)R * A, 1.f, st);
     for (int k = 0; k < S && !rc; ++k) {
         float *ik = inv + (size_t)k * N * N;
