@@ -499,6 +499,13 @@ namespace {
 // row are zero.  All times sigma.
 template <bool M> __host__ __device__ constexpr int dl_entries(int R) { return M ? R + 1 : R + 3; }
 
+// s (d + dl), dl the step's part below FP32 (of either sign, or zero: an infinite
+// sample takes d alone, which keeps its sign).
+__device__ __forceinline__ float scaled(float s, float d, float dl)
+{
+    return isfinite(s) ? fmaf(s, d, s * dl) : s * d;
+}
+
 // One CTA writes the quads of one view.  bad[view]: it holds a non-finite
 // sample.
 template <bool M>
@@ -517,7 +524,7 @@ __global__ __launch_bounds__(256) void k_dl_quads(const float *__restrict__ s_am
     auto at = [&](int n) {
         const float s = (n >= 0 && n < R && n != lost) ? __ldg(row + n) : 0.f;
         nonfinite |= (__float_as_uint(s) & 0x7F800000u) == 0x7F800000u;
-        return fmaf(s, d, s * dl);
+        return scaled(s, d, dl);
     };
     for (int e = threadIdx.x; e < dl_entries<M>(R); e += 256)
         out[e] = M ? make_float4(at(e - 1), at(e), at(R - 1 - e), at(R - e))
@@ -670,7 +677,7 @@ __device__ __noinline__ float2 dl_axis_sum(int row, int col, int nax, const DLAx
                                         : (r.ja == m ? r.wa : r.jb == m ? r.wb : 0.f);
             if (w != 0.f) {           // (the walk's entry pixels may split as 6 and -5)
                 const float s = s_am[(size_t)ax.view * R + k];
-                sum = fmaf(w, fmaf(s, ax.sigma, s * ax.sigma_lo), sum);
+                sum = fmaf(w, scaled(s, ax.sigma, ax.sigma_lo), sum);
                 den = fmaf(w, ax.sigma, den);
             }
         }
