@@ -1324,7 +1324,7 @@ int rg_radon_transpose_bresenham(rg_image sino, rg_image image, void *ws, size_t
     float *am = (float *)s.take((size_t)g.R * g.A * sizeof(float));
     float *img = (float *)s.take((size_t)g.lines * g.columns * sizeof(float));
     const float *s_am = am;
-    if (lines && is_view_major(sino))
+    if (lines && is_view_major(sino) && !overlap(sino, image))
         s_am = sino.data;
     else
         rc = launch_to_am(sino.data, sino.column_stride, sino.line_stride, g.R, g.A, am, st);
@@ -1374,7 +1374,7 @@ int rg_backprojection_bresenham(rg_image sino, rg_image image, void *ws, size_t 
     double *num = (double *)s.take(npix * sizeof(double));
     double *den = (double *)s.take(npix * sizeof(double));
     const float *s_am = am;
-    if (lines && is_view_major(sino))
+    if (lines && is_view_major(sino) && !overlap(sino, image))
         s_am = sino.data;
     else
         rc = launch_to_am(sino.data, sino.column_stride, sino.line_stride, g.R, g.A, am, st);

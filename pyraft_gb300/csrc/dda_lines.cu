@@ -436,13 +436,14 @@ __global__ __launch_bounds__(256) void k_dl_axis(const __grid_constant__ DLArgs 
 }
 
 template <int EPI>
-int radon_epi(const DLPlan &q, const DLArgs &dl, float2 *prow, float2 *pcol, float *out,
-              long long ovs, long long ors, const float *y_am, cudaStream_t st)
+int radon_epi(const DLPlan &q, const DLArgs &dl, const float *img, long long ics, long long ils,
+              float2 *prow, float2 *pcol, float *out, long long ovs, long long ors,
+              const float *y_am, cudaStream_t st)
 {
     const SSPlan &p = q.p;
     const int L = q.g.lines, C = q.g.columns, R = q.g.R;
-    RG_CK(launch_pdl(k_dl_pairs, dim3((C + 31) / 32, (L + 31) / 32), 256, 0, st, 1, dl.img, dl.ics,
-                     dl.ils, L, C, prow, pcol));
+    RG_CK(launch_pdl(k_dl_pairs, dim3((C + 31) / 32, (L + 31) / 32), 256, 0, st, 1, img, ics, ils, L,
+                     C, prow, pcol));
     RG_CK_LAUNCH("k_dl_pairs");
     if (p.nv > 0 && radon_tma_usable(p))
         return launch_radon_tma(p, prow, pcol, out, ovs, ors, y_am, R, st, 1, 0, 0, EPI, &dl);
@@ -483,9 +484,9 @@ int launch_dl_radon(const DLPlan &q, const float *img, long long ics, long long 
     s.base = (char *)scratch;
     float2 *prow = (float2 *)s.take((size_t)L * pairs_pitch(C) * sizeof(float2));
     float2 *pcol = (float2 *)s.take((size_t)C * pairs_pitch(L) * sizeof(float2));
-    const DLArgs dl = {q.g, q.d_cs, img, ics, ils, prow, pcol, q.nax, q.axis, q.rays};
-    return y_am ? radon_epi<kEpiRatio>(q, dl, prow, pcol, out, ovs, ors, y_am, st)
-                : radon_epi<kEpiSum>(q, dl, prow, pcol, out, ovs, ors, nullptr, st);
+    const DLArgs dl = {q.g, q.d_cs, prow, pcol, q.nax, q.axis, q.rays};
+    return y_am ? radon_epi<kEpiRatio>(q, dl, img, ics, ils, prow, pcol, out, ovs, ors, y_am, st)
+                : radon_epi<kEpiSum>(q, dl, img, ics, ils, prow, pcol, out, ovs, ors, nullptr, st);
 }
 
 namespace {

@@ -26,9 +26,7 @@ static_assert(sizeof(DLRay) == 32, "DLRay layout");
 struct DLArgs {
     DDAGeom g;
     const double *cs;                  // cos, sin of the views
-    const float *img;                  // the image itself, element (i, j) at i ics + j ils
-    long long ics, ils;
-    const float2 *prow, *pcol;         // its line pairs
+    const float2 *prow, *pcol;         // the image's line pairs
     int nax;
     const DLAxis *axis;
     const DLRay *rays;
@@ -37,7 +35,8 @@ struct DLArgs {
 // The ray sum of ray k of view j by the walk.  A pair's difference carries a
 // non-finite pixel to rays that only pass beside it, so every ray whose line
 // sum is not finite is walked instead: it meets the pixels that the walk
-// visits, no others.
+// visits, no others.  The walk reads the line pairs too: the image may lie in
+// memory that other CTAs store rays to by now.
 inline __device__ __noinline__ float dl_walk_ray(const DLArgs &a, int k, int j)
 {
     const DDAGeom &g = a.g;
@@ -49,7 +48,7 @@ inline __device__ __noinline__ float dl_walk_ray(const DLArgs &a, int k, int j)
     float acc = 0.f, comp = 0.f;
     dda_walk<kDdaSigma32>(it, 2 * (g.lines + g.columns) + 8, 0,
                           [&](int pi, int pj, float sg, int) {
-        const float x = __ldg(a.img + (long long)pi * a.ics + (long long)pj * a.ils) * sg;
+        const float x = __ldg(&a.prow[(size_t)pi * pairs_pitch(g.columns) + 1 + pj].x) * sg;
         const float y = x - comp, t = acc + y;
         comp = (t - acc) - y;
         acc = t;
