@@ -33,10 +33,11 @@
 // A ray through the corner where it enters the image may be lost by the walk's
 // rounding (lost_ray): the Radon walks it, the transpose leaves its sample out,
 // and the normalised backprojection of such a scan walks.
-// Plans with views between 2^-30 and 2^-14 of an axis, pixels that are not
-// square (where the walk departs from the geometry) or positions beyond 2^22
-// keep the walking kernels, and a ray whose line sum is not finite is walked
-// (dl_walk_ray).
+// Plans with views between 2^-30 and 2^-14 of an axis or with more than
+// kDlAxisMax axis-aligned ones, pixels that are not square (where the walk
+// departs from the geometry), images of more than 2097120 lines or columns (the
+// grids' limit) or positions beyond 2^22 keep the walking kernels, and a ray
+// whose line sum is not finite is walked (dl_walk_ray).
 //
 // Positions are Q24.40 (origins and steps within 2^-41 of a sample; at
 // 4096 lines and rays within 2e-9), rounded to Q9.23 once per strip or pixel
@@ -67,6 +68,11 @@ constexpr int kDlQuarter = 3;   // half-turn pairs of views and their reflection
 // The partner windows of kDlQuarter lie this far behind the views' (bytes), an
 // immediate of their loads.
 constexpr int kDlPartner = 24576;
+
+// Most axis-aligned views of a plan, which holds 32 bytes for each of their rays (a
+// scan over 2 pi has five): a scan of nothing else would hold as much as the
+// sinogram eight times over.
+constexpr int kDlAxisMax = 16;
 
 // Sums a thread keeps per row.
 __host__ __device__ constexpr int dl_sums(int form) { return form == kDlTaps ? 1 : form == kDlHalf ? 2 : 4; }
@@ -190,6 +196,7 @@ int dl_plan_build(DLPlan &q, const DDAGeom &g, const double *cs, int stride, int
         dda_set_theta(it, c, s);
         const double u = it.epsilon_update / it.delta_slow;
         if (u < 9.3132257461547852e-10) {             // 2^-30
+            if ((int)ax.size() == kDlAxisMax) return RG_OK;
             const float sg = (float)it.sigma_tilde;
             ax.push_back(DLAxis{sg, (float)(it.sigma_tilde - (double)sg), j, it.fast_is_i});
             for (int k = 0; k < R; ++k) {
@@ -465,9 +472,10 @@ int radon_epi(const DLPlan &q, const DLArgs &dl, const float *img, long long ics
 
 }  // namespace
 
+// (65535 rows of CTAs take 32 lines each)
 bool dl_sizes_ok(int L, int C, int R)
 {
-    return L >= 2 && C >= 2 && R >= 2 && (long long)L * C <= (1LL << 28) && R <= (1 << 20);
+    return L <= 65535 * 32 && C <= 65535 * 32 && L >= 2 && C >= 2 && R >= 2 && (long long)L * C <= (1LL << 28) && R <= (1 << 20);
 }
 
 size_t dl_radon_bytes(int L, int C)
