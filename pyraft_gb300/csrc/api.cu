@@ -1216,11 +1216,15 @@ static int dda_views(const DDAGeom &g, std::shared_ptr<DevTable> &out)
 // plans; a geometry they do not serve is cached too (ok false, no memory).
 struct DLHolder {
     DLPlan p;
+    std::shared_ptr<DevTable> cs;      // the views' table, which a walk in a capture finds
     ~DLHolder() { dl_plan_free(p); }
 };
 static Cache<DLHolder> g_dl_plans;
 
-static int dl_plan(const DDAGeom &g, int stride, int first, std::shared_ptr<DLHolder> &out)
+// In a stream capture, which admits no allocation, a geometry without a plan is
+// left to the walking kernels (a holder with ok false, not cached).
+static int dl_plan(const DDAGeom &g, int stride, int first, cudaStream_t st,
+                   std::shared_ptr<DLHolder> &out)
 {
     KeyBuilder kb;
     kb.add(current_device()).add(g.lines).add(g.columns).add(g.R).add(g.A).add(g.itl_x)
@@ -1230,17 +1234,26 @@ static int dl_plan(const DDAGeom &g, int stride, int first, std::shared_ptr<DLHo
     out = g_dl_plans.find(kb.s);
     if (out) return RG_OK;
     auto h = std::make_shared<DLHolder>();
-    const int rc = dl_plan_build(h->p, g, dda_cos_sin(g).data(), stride, first);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    RG_CK(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) {
+        out = h;
+        return RG_OK;
+    }
+    int rc = dda_views(g, h->cs);
+    if (!rc)
+        rc = dl_plan_build(h->p, g, dda_cos_sin(g).data(), (const double *)h->cs->p, stride, first);
     if (rc != RG_OK) return rc;
     g_dl_plans.put(kb.s, h);
     out = h;
     return RG_OK;
 }
 
-int get_dl_plan(const DDAGeom &g, int stride, int first, const DLPlan **out, void **holder)
+int get_dl_plan(const DDAGeom &g, int stride, int first, cudaStream_t st, const DLPlan **out,
+                void **holder)
 {
     std::shared_ptr<DLHolder> h;
-    const int rc = dl_plan(g, stride, first, h);
+    const int rc = dl_plan(g, stride, first, st, h);
     if (rc) return rc;
     *out = &h->p;
     *holder = new std::shared_ptr<void>(h);
@@ -1275,7 +1288,7 @@ int rg_radon_bresenham(rg_image image, rg_image sino, void *ws, size_t wsb, void
     cudaStream_t st = (cudaStream_t)stream;
     const DDAGeom g = dda_geom(image, sino);
     std::shared_ptr<DLHolder> dl;
-    if ((rc = dl_plan(g, 1, 0, dl))) return rc;
+    if ((rc = dl_plan(g, 1, 0, st, dl))) return rc;
     std::shared_ptr<DevTable> cs;
     if (!dl->p.ok && (rc = dda_views(g, cs))) return rc;
     Scratch s;
@@ -1314,7 +1327,7 @@ int rg_radon_transpose_bresenham(rg_image sino, rg_image image, void *ws, size_t
     cudaStream_t st = (cudaStream_t)stream;
     const DDAGeom g = dda_geom(image, sino);
     std::shared_ptr<DLHolder> dl;
-    if ((rc = dl_plan(g, 1, 0, dl))) return rc;
+    if ((rc = dl_plan(g, 1, 0, st, dl))) return rc;
     const bool lines = dl->p.ok && dl->p.gather;
     std::shared_ptr<DevTable> cs;
     if (!lines && (rc = dda_views(g, cs))) return rc;
@@ -1359,7 +1372,7 @@ int rg_backprojection_bresenham(rg_image sino, rg_image image, void *ws, size_t 
     cudaStream_t st = (cudaStream_t)stream;
     const DDAGeom g = dda_geom(image, sino);
     std::shared_ptr<DLHolder> dl;
-    if ((rc = dl_plan(g, 1, 0, dl))) return rc;
+    if ((rc = dl_plan(g, 1, 0, st, dl))) return rc;
     // (a ray that the walk loses has no weight here either: its four pixels
     // would need sums of weights of their own)
     const bool lines = dl->p.ok && dl->p.gather && !dl->p.lost;

@@ -164,14 +164,13 @@ void dl_plan_free(DLPlan &q)
 {
     ss_plan_free(q.p);
     if (q.d_axis) cudaFree(q.d_axis);
-    if (q.d_cs) cudaFree(q.d_cs);
     q.d_axis = nullptr;
-    q.d_cs = nullptr;
     q.ok = false;
     q.gather = 0;
 }
 
-int dl_plan_build(DLPlan &q, const DDAGeom &g, const double *cs, int stride, int first)
+int dl_plan_build(DLPlan &q, const DDAGeom &g, const double *cs, const double *d_cs, int stride,
+                  int first)
 {
     q.ok = false;
     q.gather = 0;
@@ -257,8 +256,7 @@ int dl_plan_build(DLPlan &q, const DDAGeom &g, const double *cs, int stride, int
     p.dense = fabs(dx) > 1.02 * fabs(dt);
     int rc;
     if ((rc = ensure_device_error_word())) return rc;
-    RG_CK(cudaMalloc(&q.d_cs, 2 * sizeof(double) * (size_t)g.A));
-    RG_CK(cudaMemcpy(q.d_cs, cs, 2 * sizeof(double) * (size_t)g.A, cudaMemcpyHostToDevice));
+    q.d_cs = d_cs;
     if (p.nv > 0) {
         RG_CK(cudaMalloc(&p.d_views, sizeof(View) * hv.size()));
         RG_CK(cudaMemcpy(p.d_views, hv.data(), sizeof(View) * hv.size(), cudaMemcpyHostToDevice));

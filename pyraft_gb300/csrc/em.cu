@@ -262,7 +262,7 @@ static int em_dda(const rg_image &sino, const rg_image &image, long long first, 
     for (int k = 0; k < S && !rc && (int)lines.size() == k; ++k) {
         const DLPlan *p = nullptr;
         void *h = nullptr;
-        if ((rc = get_dl_plan(g, S, k, &p, &h))) break;
+        if ((rc = get_dl_plan(g, S, k, st, &p, &h))) break;
         hold.h.push_back(h);
         if (p->ok && p->gather) lines.push_back(p);
     }

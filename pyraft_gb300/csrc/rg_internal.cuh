@@ -494,12 +494,13 @@ struct DLPlan {
     const DLRay *rays = nullptr;   // [nax][R]
     const DLAxis *axis = nullptr;  // [nax]
     const int2 *range = nullptr;   // [nax][ax_ne]: rays that meet a pixel
-    double *d_cs = nullptr;        // cos, sin of all views
+    const double *d_cs = nullptr;  // cos, sin of all views (the caller's table)
     int wg[2] = {0, 0};            // gather windows (entries) at 4 and 8 rows per thread
 };
-// cs: cos, sin of the views (host); leaves q.ok false where the line sums do
+// cs, d_cs: cos, sin of the views on host and device; leaves q.ok false where the line sums do
 // not serve.
-int dl_plan_build(DLPlan &q, const DDAGeom &g, const double *cs, int stride, int first);
+int dl_plan_build(DLPlan &q, const DDAGeom &g, const double *cs, const double *d_cs, int stride,
+                  int first);
 void dl_plan_free(DLPlan &q);
 bool dl_sizes_ok(int L, int C, int R);
 // Scratch (256-byte aligned) of the Radon and of the transpose of nv views.
@@ -518,7 +519,8 @@ int launch_dl_normalised(const DLPlan &q, const float *s_am, float *out, long lo
 int launch_dl_update(const DLPlan &q, const float *s_am, float *x, const float *inv, void *scratch,
                      cudaStream_t st);
 // The cached plan of views first, first + stride, ... (api.cu).
-int get_dl_plan(const DDAGeom &g, int stride, int first, const DLPlan **out, void **holder);
+int get_dl_plan(const DDAGeom &g, int stride, int first, cudaStream_t st, const DLPlan **out,
+                void **holder);
 // elementwise on view-major sinograms: out = max(a - b, 0) (b may be null)
 int launch_sub_clamp(const float *a, const float *b, float *out, size_t n, cudaStream_t st);
 int launch_em_update(float *x, const float *bp, const float *inv_sens, size_t n, cudaStream_t st);
