@@ -202,8 +202,9 @@ static int em_ss_core(const SSGeom &g, long long first, long long count, int S,
             const int k = (int)(j % S);
             const int kn = (int)((j + 1) % S);
             if (tiles(k)) {
-                // its epilogue clears the next subset's rows
-                const bool clear = kn != k && j + 1 < first + count && tiles(kn);
+                // its epilogue clears the next subset's rows (one grid row each)
+                const bool clear = kn != k && j + 1 < first + count && tiles(kn) &&
+                                   plans[k]->nv + plans[kn]->nv <= 65535;
                 rc = launch_radon_tiles(*plans[k], x, N, 1, 0, ratio, R, y_am, R, st, 1, 0,
                                         kEpiRatioId, k == cleared, clear ? plans[kn] : nullptr);
                 cleared = clear ? kn : -1;
