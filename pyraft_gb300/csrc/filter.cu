@@ -464,6 +464,16 @@ __global__ __launch_bounds__(kFftThreads) void k_filter_fft(const float *__restr
         }
         return r;
     };
+    // A complex transform would carry a non-finite sample of one row to the other:
+    // the lowpass forms take it as zero here; it stays in its row's sum, which
+    // makes that row NaN, as its direct sums would be.
+    auto clean = [&](float2 r) {
+        if (mode != kFilterLinear) {
+            if (!isfinite(r.x)) r.x = 0.f;
+            if (!isfinite(r.y)) r.y = 0.f;
+        }
+        return r;
+    };
     // load D, forward stage of span H.  v[i - 1] comes from the lane below
     // (lane 0 loads it); the loop runs warp-uniformly so that every lane
     // takes part in the shuffles.
@@ -471,20 +481,20 @@ __global__ __launch_bounds__(kFftThreads) void k_filter_fft(const float *__restr
     const int lane = t & 31;
     for (int ib = t - lane; ib < H; ib += kFftThreads) {
         const int i = ib + lane;
-        const float2 vi = v(i);                    // zero for i >= R (and so for i >= H)
+        const float2 raw = v(i), vi = clean(raw);  // zero for i >= R (and so for i >= H)
         float2 vp;
         vp.x = __shfl_up_sync(0xffffffffu, vi.x, 1);
         vp.y = __shfl_up_sync(0xffffffffu, vi.y, 1);
         if (i >= H) continue;
-        if (lane == 0) vp = v(i == 0 && mode != kFilterLinear ? R - 1 : i - 1);
-        s = cadd(s, vi);
+        if (lane == 0) vp = clean(v(i == 0 && mode != kFilterLinear ? R - 1 : i - 1));
+        s = cadd(s, raw);
         // wrap: R differences, none at i = R
         const float2 a = wrap && i >= R ? make_float2(0.f, 0.f) : csub(vi, vp);
         float2 c = make_float2(0.f, 0.f);
         if (!wrap && i + H <= R) {                 // circular: always; else i = 0, R = H
             const float2 vh = v(i + H);
             if (circ) s = cadd(s, vh);
-            c = csub(vh, v(i + H - 1));
+            c = csub(clean(vh), clean(v(i + H - 1)));
         }
         z[fpad(i)] = cadd(a, c);
         z[fpad(i + H)] = cmul(csub(a, c), __ldg(tw + i));
@@ -525,6 +535,10 @@ __global__ __launch_bounds__(kFftThreads) void k_filter_fft(const float *__restr
     float2 tot = make_float2(0.f, 0.f);
 #pragma unroll
     for (int w = 0; w < kFftThreads / 32; ++w) tot = cadd(tot, wsum[w]);
+    if (mode != kFilterLinear) {
+        if (!isfinite(tot.x)) tot.x -= tot.x;         // NaN
+        if (!isfinite(tot.y)) tot.y -= tot.y;
+    }
     const float dcx = tot.x * g0, dcy = tot.y * g0;
     if constexpr (QUADS) {
         // outputs n < H and n + H (circular form, R = M) read z[n] and z[n + H]
