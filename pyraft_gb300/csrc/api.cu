@@ -121,12 +121,19 @@ static size_t quads_ws(const rg_image &sino, int nz = 1)
 // Entries kept: 1024, so that a batched OSEM of many slices (slices x subsets
 // plans) finds them all again; at 64, 8 slices of 10 subsets rebuilt their 80
 // plans on every call, 2.5 ms of allocations and frees that wait for the GPU.
-// A plan holds 112 bytes per view and 4 per (64 rays, 16 views): 0.3 MB at
-// 2048 rays x 1800 views.
+// A plan holds 0.3 MB at 2048 rays x 1800 views, so that 1024 fit the bound in
+// bytes, which the lists of axis-aligned rays of DDA scans (100 MB for a million
+// rays) would exceed by far; the newest entry is always kept.
 template <class T>
 struct Cache {
-    using Item = std::pair<std::string, std::shared_ptr<T>>;
+    struct Item {
+        std::string first;
+        std::shared_ptr<T> second;
+        size_t bytes;
+    };
     std::mutex mu;
+    size_t held = 0;         // device bytes of the entries
+    static constexpr size_t kBytes = (size_t)384 << 20;
     std::list<Item> items;   // MRU first
     std::unordered_map<std::string, typename std::list<Item>::iterator> index;
     size_t cap = 1024;
@@ -137,11 +144,13 @@ struct Cache {
         items.splice(items.begin(), items, it->second);
         return items.front().second;
     }
-    void put(const std::string &k, std::shared_ptr<T> v)
+    void put(const std::string &k, std::shared_ptr<T> v, size_t bytes)
     {
-        items.emplace_front(k, std::move(v));
+        items.push_front(Item{k, std::move(v), bytes});
         index[k] = items.begin();
-        while (items.size() > cap) {
+        held += bytes;
+        while (items.size() > cap || (held > kBytes && items.size() > 1)) {
+            held -= items.back().bytes;
             index.erase(items.back().first);
             items.pop_back();
         }
@@ -198,6 +207,14 @@ struct PlanHolder {
 
 static Cache<PlanHolder> g_plans;
 
+// Device bytes of a plan: its views (twice, for the tile-driven Radon), and the
+// TMA Radon's blocks and CTA order.
+static size_t plan_bytes(const SSPlan &p)
+{
+    return (size_t)p.nv * (sizeof(View) + sizeof(TtView)) +
+           (size_t)p.nblocks * (16 + 8 * (size_t)((p.g.R + 63) / 64));
+}
+
 // Plan over views {first, first + stride, ...} of the geometry.
 static int get_plan(const SSGeom &g, int stride, int first, std::shared_ptr<PlanHolder> &out)
 {
@@ -212,7 +229,7 @@ static int get_plan(const SSGeom &g, int stride, int first, std::shared_ptr<Plan
     auto h = std::make_shared<PlanHolder>();
     int rc = ss_plan_build(h->p, g, views.data(), (int)views.size());
     if (rc != RG_OK) return rc;
-    g_plans.put(kb.s, h);
+    g_plans.put(kb.s, h, plan_bytes(h->p));
     out = h;
     return RG_OK;
 }
@@ -239,7 +256,7 @@ static int get_table(const std::string &key, const void *host, size_t bytes,
     auto t = std::make_shared<DevTable>();
     RG_CK(cudaMalloc(&t->p, bytes));
     RG_CK(cudaMemcpy(t->p, host, bytes, cudaMemcpyHostToDevice));
-    g_tables.put(kb.s, t);
+    g_tables.put(kb.s, t, bytes);
     out = t;
     return RG_OK;
 }
@@ -261,7 +278,7 @@ static int get_table_lazy(const std::string &key, F fill, std::shared_ptr<DevTab
     fill(host, *t);
     RG_CK(cudaMalloc(&t->p, host.size()));
     RG_CK(cudaMemcpy(t->p, host.data(), host.size(), cudaMemcpyHostToDevice));
-    g_tables.put(kb.s, t);
+    g_tables.put(kb.s, t, host.size());
     out = t;
     return RG_OK;
 }
@@ -1244,7 +1261,7 @@ static int dl_plan(const DDAGeom &g, int stride, int first, cudaStream_t st,
     if (!rc)
         rc = dl_plan_build(h->p, g, dda_cos_sin(g).data(), (const double *)h->cs->p, stride, first);
     if (rc != RG_OK) return rc;
-    g_dl_plans.put(kb.s, h);
+    g_dl_plans.put(kb.s, h, plan_bytes(h->p.p) + dl_axis_bytes(h->p));
     out = h;
     return RG_OK;
 }

@@ -169,6 +169,11 @@ void dl_plan_free(DLPlan &q)
     q.gather = 0;
 }
 
+size_t dl_axis_bytes(const DLPlan &q)
+{
+    return (size_t)q.nax * (sizeof(DLAxis) + sizeof(DLRay) * (size_t)q.g.R + sizeof(int2) * (size_t)q.ax_ne);
+}
+
 int dl_plan_build(DLPlan &q, const DDAGeom &g, const double *cs, const double *d_cs, int stride,
                   int first)
 {

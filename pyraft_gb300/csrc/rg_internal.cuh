@@ -502,6 +502,7 @@ struct DLPlan {
 int dl_plan_build(DLPlan &q, const DDAGeom &g, const double *cs, const double *d_cs, int stride,
                   int first);
 void dl_plan_free(DLPlan &q);
+size_t dl_axis_bytes(const DLPlan &q);    // device bytes of the axis-aligned views' lists
 bool dl_sizes_ok(int L, int C, int R);
 // Scratch (256-byte aligned) of the Radon and of the transpose of nv views.
 size_t dl_radon_bytes(int L, int C);

@@ -49,3 +49,20 @@ def test_scan_of_axis_aligned_views_keeps_no_ray_lists(orc):
     assert grown < 32 << 20
     ref = orc.radon_bresenham(x.astype(np.float64), r, 2, (-1.0, 1.0, 1.0, -1.0), sc)
     assert rel(got[:, [0, 999, 1999]], ref[:, [0, 0, 0]]) <= 4e-7
+
+
+def test_cached_plans_are_bounded_in_bytes():
+    """24 scans of 400000 rays with three axis-aligned views, whose lists take 38 MB
+    each: the cache of plans keeps 384 MB."""
+    r, n = 400000, 16
+    g = rg.gpu_image(torch.ones((n, n), device="cuda"), (-1.0, 1.0), (1.0, -1.0))
+    run = lambda e: rg.radon(g, (r, 3), DDA, top_left=(0.0, e), bottom_right=(math.pi, -e)).data
+    run(1.0)
+    torch.cuda.synchronize()
+    free, held = torch.cuda.mem_get_info()[0], torch.cuda.memory_reserved()
+    for k in range(24):
+        out = run(1.0 + 0.01 * k)
+    torch.cuda.synchronize()
+    grown = free - torch.cuda.mem_get_info()[0] - (torch.cuda.memory_reserved() - held)
+    assert grown <= 400 << 20
+    assert bool((out.sum(0) > 0).all())
