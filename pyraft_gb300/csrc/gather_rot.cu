@@ -821,15 +821,16 @@ int gather_rot_tma(const SSPlan &p, const float *s_am, int s_ld, float *out, lon
 
 // Whether the paired gathers of nz slices stage by TMA where the call brings the
 // quad scratch (RG_GATHER_ROT_TMA: 0 never, 1 always).  From 256 view pairs
-// always.  Below, by the work (pixels x pairs), loads / TMA in us: the prepass
-// must be made up for.  Adjoint 512^2 x 180 pairs 48.1
-// / 49.0, x 250 61.3 / 59.5, 1024^2 x 90 78.8 / 76.0, x 180 137 / 126, 2048^2 x
-// 180 463 / 416, a stack of 8 512^2 x 180 294 / 273 (x 90 168 / 171).
-// Backprojection 512^2 x 180 48 / 46, 1024^2 x 180 121 / 126, x 250 159 / 161,
-// 2048^2 x 180 402 / 376.  In the FBP the filter writes the quads and zeroes the
-// image (`prefilled`), which saves a launch: 128^2 x 32 35.2 / 29.1, 256^2 x 90
-// 31.7 / 27.3, 256^2 x 180 36.2 / 36.1, 512^2 x 90 38.2 / 39.3, 1024^2 x 180 129 /
-// 134, 2048^2 x 180 414 / 397.
+// always.  Below, the adjoint stages by loads: TMA is up to 8 % faster on one
+// image (1024^2 x 180 pairs 133 / 122 us) and 1 % on a stack (a gradient step of 8
+// images 512^2 x 180 pairs 550 / 543 us), but the tuner then takes shapes with
+// longer FP32 sums (2.65e-7 -> 2.97e-7 from 64 bits on that step).  The
+// backprojection goes by the work (pixels x pairs), loads / TMA in us, as the
+// prepass must be made up for: 512^2 x 180 48 / 46, 1024^2 x 180 121 / 126, x 250
+// 159 / 161, 2048^2 x 180 402 / 376; in the FBP the filter writes the quads and
+// zeroes the image (`prefilled`), which saves a launch: 128^2 x 32 35.2 / 29.1,
+// 256^2 x 90 31.7 / 27.3, 256^2 x 180 36.2 / 36.1, 512^2 x 90 38.2 / 39.3, 1024^2 x
+// 180 129 / 134, 2048^2 x 180 414 / 397.
 bool gather_rot_use_tma(const SSPlan &p, int mode, int nz, bool prefilled)
 {
     const char *e = getenv("RG_GATHER_ROT_TMA");
@@ -837,8 +838,8 @@ bool gather_rot_use_tma(const SSPlan &p, int mode, int nz, bool prefilled)
     if (e && !strcmp(e, "1")) return true;
     const int pairs = p.nv / 2;
     if (pairs >= kTmaMinPairs) return true;
+    if (mode == 1) return false;
     const double work = (double)nz * p.g.N * p.g.N * pairs;
-    if (mode == 1) return pairs >= 128 ? work >= 64e6 : pairs >= 90 && nz == 1 && work >= 90e6;
     return (prefilled && work <= 11e6) || (pairs >= 128 && work >= 700e6);
 }
 
