@@ -19,8 +19,8 @@
 // GB300: Radon 25.0 -> 2.30 ms (issue-bound, as the slant-stack's), transpose
 // 28.0 -> 2.05 ms (74 % of the shared-memory rate); 1024^2 x 720: 2.73 ->
 // 0.26 and 3.2 -> 0.25 ms.  The normalised backprojection (A^T s / A^T 1, two
-// FP64 atomics a pixel in the walk) sums both with compensation in the same
-// gather: 68.9 -> 3.8 ms, 512^2 x 360 1.11 -> 0.10 ms.  Error against 64 bits
+// FP64 atomics a pixel in the walk) keeps both sums in two FP32 numbers in the
+// same gather: 68.8 -> 6.4 ms, 512^2 x 360 1.11 -> 0.14 ms.  Error against 64 bits
 // (rel-L2): Radon 4.1e-8 -> 2.6e-8, transpose 4.4e-7 -> 8e-8, normalised 2.5e-8
 // (the rounding of its result) as before.
 //
@@ -520,7 +520,7 @@ __device__ __forceinline__ float scaled(float s, float d, float dl)
 
 // One CTA writes the quads of one view.  bad[view]: it holds a non-finite
 // sample.
-template <bool M>
+template <bool M, bool RAW>
 __global__ __launch_bounds__(256) void k_dl_quads(const float *__restrict__ s_am, int R,
                                                   const View *__restrict__ views,
                                                   float4 *__restrict__ quads,
@@ -536,7 +536,7 @@ __global__ __launch_bounds__(256) void k_dl_quads(const float *__restrict__ s_am
     auto at = [&](int n) {
         const float s = (n >= 0 && n < R && n != lost) ? __ldg(row + n) : 0.f;
         nonfinite |= (__float_as_uint(s) & 0x7F800000u) == 0x7F800000u;
-        return scaled(s, d, dl);
+        return RAW ? s : scaled(s, d, dl);
     };
     for (int e = threadIdx.x; e < dl_entries<M>(R); e += 256)
         out[e] = M ? make_float4(at(e - 1), at(e), at(R - 1 - e), at(R - e))
@@ -553,7 +553,7 @@ struct __align__(16) DLSlot {
     unsigned step;
     float P, c0;
     int state;          // -1: skip, 0, else CAREFUL (non-finite samples, detector's end)
-    float sigma;        // NORM: (base is not rounded, P is times 2^-30)
+    float sigma, sigma_lo;   // NORM: (base is not rounded, P is times 2^-30)
     int nlo;            // NORM: first entry's ray
     int half;           // NORM: where the trapezoid is at half its height (Q2.30)
 };
@@ -567,15 +567,18 @@ __device__ __forceinline__ float4 lds_quad(unsigned addr)
     return q;
 }
 
-// kahan_add that leaves an infinite sum infinite.
-__device__ __forceinline__ void kahan_add_inf(float &sum, float &c, float x)
+// sum - c += a (w + wl), the product and the sum with their rounding errors (of
+// the first terms, larger than the sum, to within an ulp of theirs): two FP32
+// numbers that do what the walks' FP64 sums do.
+__device__ __forceinline__ void dot_add(float &sum, float &c, float a, float w, float wl)
 {
-    kahan_add(sum, c, x);
-    if (!isfinite(c)) c = 0.f;
+    const float p = a * w, e = fmaf(a, wl, fmaf(a, w, -p)), t = sum + p;
+    c -= (p - (t - sum)) + e;
+    sum = t;
 }
 
-// Sums of a thread.  NORM (the normalised backprojection): every sum is
-// compensated, and den sums the weights.  The reflected view at the
+// Sums of a thread.  NORM (the normalised backprojection): every sum comes with
+// its rounding errors, and den sums the weights.  The reflected view at the
 // reflected pixel and the half-turn mirror have the pixel's weights, so one
 // sum of weights serves them all.
 template <int F, int ROWS, bool NORM>
@@ -595,7 +598,12 @@ struct DLSums {
 // trapezoid's half height in Q2.30 (an integer subtraction and a conversion
 // more each): its quotients are rounded once, and the position's rounding
 // would show beside that (512^2 x 360: 2.6e-8 against 2.45e-8 for the rounding
-// alone, 300^2 x 200 2.9e-8 against 2.5e-8).
+// alone, 300^2 x 200 2.9e-8 against 2.5e-8).  So would one rounding of every
+// product, of the samples times sigma or of sigma (2.518e-8 and 2.532e-8 against
+// 2.501e-8 for the rounding alone, which the walk's FP64 sums reach): the
+// samples stay as they are, sigma goes with the weights in two parts, and the
+// products keep their rounding errors: 2.502e-8 and 2.503e-8, 512^2 x 360 100 ->
+// 143 us (the walk 1115).
 template <int F, int ROWS, bool CAREFUL, bool NORM>
 __device__ __forceinline__ void dl_slot(long long pos, const DLSlot &si, unsigned pw,
                                         unsigned quad_bytes, int R, DLSums<F, ROWS, NORM> &t)
@@ -610,12 +618,16 @@ __device__ __forceinline__ void dl_slot(long long pos, const DLSlot &si, unsigne
         if (CAREFUL) return w > 0.f ? fmaf(v, w, sum) : sum;
         return fmaf(v, w, sum);
     };
-    // sum i of row r: + a wa + b wb
-    auto add2 = [&](int i, int r, float a, float wa, float b, float wb) {
-        if constexpr (NORM && CAREFUL)
-            kahan_add_inf(t.s[i][r], t.c[i][r], term(term(0.f, a, wa), b, wb));
-        else if constexpr (NORM) kahan_add(t.s[i][r], t.c[i][r], term(term(0.f, a, wa), b, wb));
-        else t.s[i][r] = term(term(t.s[i][r], a, wa), b, wb);
+    // sum i of row r: + a wa + b wb (NORM: wa, wb with their lower parts la, lb)
+    auto add2 = [&](int i, int r, float a, float wa, float b, float wb, float la, float lb) {
+        if constexpr (NORM) {
+            float &s = t.s[i][r], &c = t.c[i][r];
+            if (!CAREFUL || wa > 0.f) dot_add(s, c, a, wa, la);
+            if (!CAREFUL || wb > 0.f) dot_add(s, c, b, wb, lb);
+            if (CAREFUL && !isfinite(c)) c = 0.f;     // an infinite sum stays infinite
+        } else {
+            t.s[i][r] = term(term(t.s[i][r], a, wa), b, wb);
+        }
     };
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
@@ -647,24 +659,39 @@ __device__ __forceinline__ void dl_slot(long long pos, const DLSlot &si, unsigne
             if ((unsigned)(k - 1) >= (unsigned)R) wz = 0.f;
             if ((unsigned)(k + 2) >= (unsigned)R) wd = 0.f;
         }
+        float la = 0.f, lb = 0.f, lz = 0.f, ld = 0.f;
+        if constexpr (NORM) {                         // the step goes with the weights
+            auto step = [&](float &w, float &l) {
+                const float v = w * si.sigma;
+                l = fmaf(w, si.sigma_lo, fmaf(w, si.sigma, -v));
+                w = v;
+                const float n = t.den[r] + v;
+                t.dc[r] -= (v - (n - t.den[r])) + l;
+                t.den[r] = n;
+            };
+            step(wa, la);
+            step(wb, lb);
+            if constexpr (F == kDlTaps) {
+                step(wz, lz);
+                step(wd, ld);
+            }
+        }
         if constexpr (F == kDlTaps) {
             if constexpr (NORM) {
-                add2(0, r, q.x, wz, q.y, wa);
-                add2(0, r, q.z, wb, q.w, wd);
+                add2(0, r, q.x, wz, q.y, wa, lz, la);
+                add2(0, r, q.z, wb, q.w, wd, lb, ld);
             } else {
                 t.s[0][r] = term(term(term(term(t.s[0][r], q.x, wz), q.y, wa), q.z, wb), q.w, wd);
             }
         } else {
-            add2(0, r, q.x, wa, q.y, wb);
-            add2(1, r, q.w, wa, q.z, wb);
+            add2(0, r, q.x, wa, q.y, wb, la, lb);
+            add2(1, r, q.w, wa, q.z, wb, la, lb);
         }
         if constexpr (F == kDlQuarter) {
             const float4 p = lds_quad<kDlPartner>(addr);
-            add2(2, r, p.x, wa, p.y, wb);
-            add2(3, r, p.w, wa, p.z, wb);
+            add2(2, r, p.x, wa, p.y, wb, la, lb);
+            add2(3, r, p.w, wa, p.z, wb, la, lb);
         }
-        if constexpr (NORM)
-            kahan_add(t.den[r], t.dc[r], si.sigma * (F == kDlTaps ? (wz + wa) + (wb + wd) : wa + wb));
         if constexpr (NORM) pos += 4 * si.row;
         else vpos += si.step;
     }
@@ -805,7 +832,7 @@ __global__ __launch_bounds__(256) void k_dl_gather(
     auto issue = [&](int c) {
         const int chunk = vbeg + c * nslots;
         const int n = min(nslots, vend - chunk), b = c & 1;
-        DLSlot si = {0, 0, 0, 0u, 0.f, 0.f, -1, 0.f, 0, 0};
+        DLSlot si = {0, 0, 0, 0u, 0.f, 0.f, -1, 0.f, 0.f, 0, 0};
         int nlo = 0;
         if (lane < n) {
             const View &v = views[chunk + lane];
@@ -832,6 +859,7 @@ __global__ __launch_bounds__(256) void k_dl_gather(
                     si.base = origin - ((long long)nlo << kDlQ);
                     si.P = v.P * 9.31322574615478515625e-10f;
                     si.sigma = v.delta;
+                    si.sigma_lo = v.delta_lo;
                     si.nlo = nlo;
                     si.half = (int)v.b0;
                     if (any_bad || nlo < 1 || (int)(mx >> kDlQ) + 3 >= R) si.state |= 2;
@@ -1013,7 +1041,7 @@ int gather_rows(const DLPlan &q, const float *s_am, const DLOut &o, float4 *quad
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS)
             return set_error(RG_ECUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-        RG_CK(launch_pdl(k_dl_quads<kMirror>, dim3(p.nv), 256, 0, st, 1, s_am, R, p.d_views, quads,
+        RG_CK(launch_pdl(k_dl_quads<kMirror, EP == kDlNorm>, dim3(p.nv), 256, 0, st, 1, s_am, R, p.d_views, quads,
                          bad));
         RG_CK_LAUNCH("k_dl_quads");
     }
