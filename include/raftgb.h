@@ -211,7 +211,9 @@ int rg_radon_slantstack_withmesh(rg_image phantom, long long phantom_stride, rg_
  *   raft/raft_filter.cpp:184, bound at pyraft/raftypes.py:185).
  * kind RG_FILTER_LOWPASS: the cosine-windowed ramp of pyraft's
  *   lowpassino_fbp (pyraft/filters/filters.py:13-68), applied as the
- *   equivalent circular convolution.
+ *   equivalent circular convolution.  A non-finite sample makes its view NaN
+ *   and no other; views that share a transform round with the larger one's
+ *   error (1e-7 of it).
  * in and out: nrays x nviews; may be the same image.                        */
 #define RG_FILTER_RAMLAK  1
 #define RG_FILTER_LOWPASS 2
@@ -237,8 +239,8 @@ int rg_fbp(rg_image sino, rg_image image, int kind,
  * nsubsets == 1 is plain EM; > 1 is OSEM over interleaved view subsets
  * (subset s = views s, s+S, s+2S, ...).  Guards: y/0 -> 0, and pixels with
  * zero sensitivity are set to 0 (the reference divides by zero).
- * The sensitivity A^T 1 is summed with compensation, its positions rounded as
- * the adjoint's.
+ * The slant stack's sensitivity A^T 1 is summed with compensation, its
+ * positions rounded as the adjoint's; the DDA's is a transpose of ones.
  * RG_BRESENHAM with niter >= 2 on a geometry that walks (pixels that are not
  * square, views 2^-30 to 2^-14 from an axis) also allocates, outside the
  * workspace, device memory for the rays' walks recorded once and replayed

@@ -1101,12 +1101,12 @@ size_t rg_fbp_workspace(rg_image sino, rg_image image, int kind)
 
 }  // extern "C"
 namespace rg {
-// RG_FBP_QUADS=0 (read per call) keeps the FBP's filter and the gather's quad
-// prepass as separate launches: the reference arrangement for tests, which
-// must give the same bits.
 // Largest ray-major sinogram that the FBP's filter reads where it lies.
 constexpr size_t kFbpDirectMax = 1 << 18;
 
+// RG_FBP_QUADS=0 (read per call) keeps the FBP's filter and the gather's quad
+// prepass as separate launches: the reference arrangement for tests, which
+// must give the same bits where both transform the same pairs of rows.
 static bool fbp_quads_enabled()
 {
     const char *e = getenv("RG_FBP_QUADS");

@@ -267,7 +267,7 @@ struct BatchRun {
     int n = 0, S = 0, wmax = 64, vpt = 2;
     bool tiles = false;               // tile-driven Radon (else the direct walks)
     int total[8][64] = {};            // [kind][subset] item counts (subset 0 for pairs)
-    int grid[5][64] = {};             // persistent grids: pairs, radon[s], -, -, tiles
+    int grid[3][64] = {};             // persistent grids: pairs, radon[s], tiles
     BatchSlice *d_desc = nullptr;     // S x n descriptors (device, in scratch)
     int *counter = nullptr;
 };
@@ -278,7 +278,7 @@ int prepare_grids(BatchRun &br)
     if (int rc = persistent_grid(k_batch_pairs, 256, 0, br.total[kLP][0], &br.grid[0][0])) return rc;
     if (br.tiles)
         if (int rc = persistent_grid(k_batch_tiles, 256, (size_t)kBtLines * kTtRowB * 8,
-                                     br.total[kTiles][0], &br.grid[4][0]))
+                                     br.total[kTiles][0], &br.grid[2][0]))
             return rc;
     for (int s = 0; s < br.S; ++s)
         if (int rc = persistent_grid(br.vpt == 2 ? k_batch_radon<2> : k_batch_radon<1>, 128, 0,
@@ -302,7 +302,7 @@ int enqueue_iteration(const BatchRun &br, cudaStream_t st)
             k_batch_rows<true><<<br.total[kRows][s], 256, 0, st>>>(d, br.n);
             RG_CK_LAUNCH("k_batch_rows (zero)");
             RG_CK(cudaMemsetAsync(br.counter, 0, sizeof(int), st));
-            k_batch_tiles<<<br.grid[4][0], 256, (size_t)kBtLines * kTtRowB * 8, st>>>(
+            k_batch_tiles<<<br.grid[2][0], 256, (size_t)kBtLines * kTtRowB * 8, st>>>(
                 d, br.n, br.total[kTiles][0], br.counter, device_error_word(),
                 (unsigned)sizeof(float2));
             RG_CK_LAUNCH("k_batch_tiles");

@@ -75,7 +75,10 @@ constexpr int kDlPartner = 24576;
 constexpr int kDlAxisMax = 16;
 
 // Sums a thread keeps per row.
-__host__ __device__ constexpr int dl_sums(int form) { return form == kDlTaps ? 1 : form == kDlHalf ? 2 : 4; }
+__host__ __device__ constexpr int dl_sums(int form)
+{
+    return form == kDlTaps ? 1 : form == kDlHalf ? 2 : 4;
+}
 
 bool to_q40(double v, long long &out)
 {
@@ -171,7 +174,8 @@ void dl_plan_free(DLPlan &q)
 
 size_t dl_axis_bytes(const DLPlan &q)
 {
-    return (size_t)q.nax * (sizeof(DLAxis) + sizeof(DLRay) * (size_t)q.g.R + sizeof(int2) * (size_t)q.ax_ne);
+    return (size_t)q.nax * (sizeof(DLAxis) + sizeof(DLRay) * (size_t)q.g.R +
+                            sizeof(int2) * (size_t)q.ax_ne);
 }
 
 int dl_plan_build(DLPlan &q, const DDAGeom &g, const double *cs, const double *d_cs, int stride,
@@ -478,7 +482,8 @@ int radon_epi(const DLPlan &q, const DLArgs &dl, const float *img, long long ics
 // (65535 rows of CTAs take 32 lines each)
 bool dl_sizes_ok(int L, int C, int R)
 {
-    return L <= 65535 * 32 && C <= 65535 * 32 && L >= 2 && C >= 2 && R >= 2 && (long long)L * C <= (1LL << 28) && R <= (1 << 20);
+    return L >= 2 && L <= 65535 * 32 && C >= 2 && C <= 65535 * 32 && R >= 2 && R <= (1 << 20) &&
+           (long long)L * C <= (1LL << 28);
 }
 
 size_t dl_radon_bytes(int L, int C)

@@ -452,8 +452,7 @@ __global__ __launch_bounds__(kFftThreads) void k_filter_fft(const float *__restr
     const bool two = pair || a0 + 1 < A;
     const float *__restrict__ x = in + a0 * ivs;
     // the second row, read only when `two`
-    const float *__restrict__ y =
-        in + (pair ? a0 + fq.roff : a0 + 1) * ivs;
+    const float *__restrict__ y = in + (pair ? a0 + fq.roff : a0 + 1) * ivs;
 
     // v[n] for n in [0, R), else 0
     auto v = [&](int n) {
@@ -585,8 +584,8 @@ __global__ __launch_bounds__(kFftThreads) void k_filter_fft(const float *__restr
     }
 }
 
-int launch_filter_fft(const float *in, long long ivs, long long irs, float *out_am, int R, int A, int p, const float2 *d_tab,
-                      float g0, int mode, cudaStream_t st)
+int launch_filter_fft(const float *in, long long ivs, long long irs, float *out_am, int R, int A,
+                      int p, const float2 *d_tab, float g0, int mode, cudaStream_t st)
 {
     if (p < 2 || p > kFilterFftMaxLog ||
         (mode == kFilterCirc ? (1 << p) != R : (1 << p) < 2 * R - 1))
@@ -600,10 +599,10 @@ int launch_filter_fft(const float *in, long long ivs, long long irs, float *out_
     return RG_OK;
 }
 
-int launch_filter_fft_quads(const float *in, long long ivs, long long irs, int R, int A, int p, const float2 *d_tab, float g0,
-                            int mode, const View *d_views, int pairs, int roff,
-                            float4 *quads, float *out, int N, long long cs, long long ls,
-                            cudaStream_t st, bool near)
+int launch_filter_fft_quads(const float *in, long long ivs, long long irs, int R, int A, int p,
+                            const float2 *d_tab, float g0, int mode, const View *d_views,
+                            int pairs, int roff, float4 *quads, float *out, int N, long long cs,
+                            long long ls, cudaStream_t st, bool near)
 {
     if (near && (2 * roff != A || pairs != roff))
         return set_error(RG_EINVAL, "filter quads: %d views do not pair by halves", A);
@@ -617,7 +616,8 @@ int launch_filter_fft_quads(const float *in, long long ivs, long long irs, int R
     RG_CK(cudaFuncSetAttribute(k_filter_fft<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)smem));
     RG_CK(launch_pdl(k_filter_fft<true>, pairs, kFftThreads, smem, st, 1, in, ivs, irs, nullptr,
-                     R, A, p, d_tab, g0, mode, FilterQuads{d_views, roff, near, quads, out, N, cs, ls}));
+                     R, A, p, d_tab, g0, mode,
+                     FilterQuads{d_views, roff, near, quads, out, N, cs, ls}));
     RG_CK_LAUNCH("k_filter_fft");
     return RG_OK;
 }

@@ -453,16 +453,16 @@ int launch_ramlak_rows(const float *in_am, float *out_am, int R, int A, const fl
 // entries); g0 = what the sum of the row adds to every output.
 constexpr int kFilterFftMaxLog = 14;
 enum { kFilterLinear = 0, kFilterCirc = 1, kFilterWrap = 2 };
-int launch_filter_fft(const float *in, long long ivs, long long irs, float *out_am, int R, int A, int p, const float2 *d_tab,
-                      float g0, int mode, cudaStream_t st);
+int launch_filter_fft(const float *in, long long ivs, long long irs, float *out_am, int R, int A,
+                      int p, const float2 *d_tab, float g0, int mode, cudaStream_t st);
 // The same filter for the FBP: CTA j filters rows v = d_views[j].view and v +
 // roff of in (j < pairs; near: rows 2j and 2j + 1) and writes the paired
 // backprojection's quads[j][e] (e < R - 1) instead of the rows, and the CTAs
 // zero the N x N output (strides cs, ls).
-int launch_filter_fft_quads(const float *in, long long ivs, long long irs, int R, int A, int p, const float2 *d_tab, float g0,
-                            int mode, const View *d_views, int pairs, int roff,
-                            float4 *quads, float *out, int N, long long cs, long long ls,
-                            cudaStream_t st, bool near);
+int launch_filter_fft_quads(const float *in, long long ivs, long long irs, int R, int A, int p,
+                            const float2 *d_tab, float g0, int mode, const View *d_views,
+                            int pairs, int roff, float4 *quads, float *out, int N, long long cs,
+                            long long ls, cudaStream_t st, bool near);
 
 // bresenham.cu
 struct DDAGeom {

@@ -72,7 +72,7 @@ def make_em(sino, shape, projection_method=radon_method.BRESENHAM,
     the slant-stack backprojection B in place of A^T)."""
     if weight is not None:
         raise TypeError('a precomputed weight is not supported; the sensitivity is computed '
-                        'on the device in FP64')
+                        'on the device')
     m = _method(projection_method, backprojection_method, reference)
     gs, _ = to_gpu(sino, (0.0, 1.0), (numpy.pi, -1.0))
 
