@@ -610,13 +610,12 @@ static int radon_rpl()
 
 // Cluster size of the strip split for a grid of `ctas` CTAs at `slots`
 // resident CTAs.  Measured on GB300 (slant-stack Radon, GUPS, split 1 / 2 / 4;
-// waves of the unsplit grid): 2048^2 x 1800 (8.1) 3713 / 3702 / 3520; 1024^2 x
-// 720 (1.6) 3211 / 3287 / 3111; 975^2, 886 rays x 621 (1.2) 2931 / 3095 / 2984;
-// 512^2 x 360 (0.4) 1167 / 1945 / 2062; 256^2 x 180 (0.1) 481 / 683 / 744.  Each
-// rank repeats the CTA's set-up and the ranks' partials meet in distributed
-// shared memory, so a split pays only where the unsplit grid leaves SMs idle:
-// 1 from 2.5 waves up, 2 from one wave, else 4, with at least 4 strips of
-// kTmLines lines per rank.
+// waves of the unsplit grid): 2048^2 x 1800 (8.1) 3997 / 3960 / 3725; 1024^2 x
+// 720 (1.6) 3410 / 3458 / 3212; 975^2, 886 rays x 621 (1.2) 3082 / 3255 / 3071;
+// 512^2 x 360 (0.4) 1211 / 1992 / 2052.  Each rank repeats the CTA's set-up and
+// the ranks' partials meet in distributed shared memory, so a split pays only
+// where the unsplit grid leaves SMs idle: 1 from 2.5 waves up, 2 from one wave,
+// else 4, with at least 4 strips of kTmLines lines per rank.
 // RG_RADON_SPLIT_TMA=1|2|4 forces it.
 static int tma_pick_split(long long ctas, int slots, int N)
 {
